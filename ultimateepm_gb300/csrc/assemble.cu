@@ -654,6 +654,17 @@ template void launch_assemble_ds<ds4>(const DevParams&, const DevParamsDS&, cons
                                       const cx<double>*, const double2*, const double*, ds4*, int, size_t, cx<float>*,
                                       size_t, int, cudaStream_t);
 
+template <typename SO>
+struct QuatOf {
+    using type = qt<double>;
+};
+template <>
+struct QuatOf<ds4> {
+    using type = qt<float>;
+};
+__device__ __forceinline__ cx<double> quat_part(cx<double> v) { return v; }
+__device__ __forceinline__ cx<float>  quat_part(ds4 v) { return mk(v.rhi, v.ihi); }
+
 // With spin-orbit coupling: the same tiling over the scalar problem's lower triangle. Each scalar
 // element (i, j), i >= j, yields four blocks' elements, UU(i, j) = h + s00, DD(i, j) = h + s11,
 // DU(i, j) = s10 and UD(i, j) = s01 (i > j), written directly at (i, j), (i + N, j + N), (i + N, j)
@@ -663,7 +674,10 @@ template void launch_assemble_ds<ds4>(const DevParams&, const DevParamsDS&, cons
 // DSM (the mixed path, SO = ds2 / ds4): the four values in double-single arithmetic on the FP32
 // pipe from the FP32-pair tables (Vloc32, phNL32, phSO32) and rows32, the nonlocal part by
 // nl_element_ds, and the FP64 element where that one routes an element to FP64.
-template <bool NL, bool DSM, typename SO>
+// QUAT: the matrix is quaternionic (DD = conj UU, DU = -conj UD exactly: spin-orbit without an
+// antisymmetric part), and UU + UD j goes to HQ (order N): with DSM the FP32 lower triangle beside H,
+// else (FP64) the full matrix in place of H.
+template <bool NL, bool DSM, bool QUAT, typename SO>
 __global__ void __launch_bounds__(256) k_assemble_soc_tiles(const DevParams P, const cx<double>* __restrict__ Vloc,
                                                             const double2* __restrict__ phNL,
                                                             const double2* __restrict__ phSO, const double* __restrict__ rows,
@@ -671,7 +685,8 @@ __global__ void __launch_bounds__(256) k_assemble_soc_tiles(const DevParams P, c
                                                             typename Lower<SO>::type* __restrict__ H32,
                                                             size_t mstride32, int batch, const DevParamsDS Q,
                                                             const float4* __restrict__ Vloc32, const float4* __restrict__ phNL32,
-                                                            const float4* __restrict__ phSO32, const float2* __restrict__ rows32) {
+                                                            const float4* __restrict__ phSO32, const float2* __restrict__ rows32,
+                                                            typename QuatOf<SO>::type* __restrict__ HQ, size_t mstrideq) {
     using SF = typename Lower<SO>::type;
     extern __shared__ __align__(16) unsigned char smraw[];
     SO(*tile)[32][33] = reinterpret_cast<SO(*)[32][33]>(smraw);  // [4][jl][il]: UU, DD, DU, UD of h(i, j)
@@ -739,6 +754,16 @@ __global__ void __launch_bounds__(256) k_assemble_soc_tiles(const DevParams P, c
                 du = stored(Hb, sv[2]);
                 ud = stored(Hb, sv[1]);
             }
+            if constexpr (QUAT) {
+                using Q1 = typename QuatOf<SO>::type;
+                const auto u = quat_part(uu), d = quat_part(ud);
+                stc(HQ + (size_t)b * mstrideq + (size_t)j * N + i, Q1{u.x, u.y, d.x, d.y});
+                if constexpr (!DSM) {
+                    tile[0][jl][tx] = uu;
+                    tile[3][jl][tx] = ud;
+                    continue;
+                }
+            }
             put(i, j, uu);
             put(i + N, j + N, dd);
             put(i + N, j, du);
@@ -756,6 +781,13 @@ __global__ void __launch_bounds__(256) k_assemble_soc_tiles(const DevParams P, c
     for (int q = 0; q < 4; ++q) {
         // mirrors: threads run down the rows j (coalesced down column i, i + N)
         const int il = ty + 8 * q, j = tj * 32 + tx, i = ti * 32 + il;
+        if constexpr (QUAT && !DSM) {
+            if (i < N && j < N && i > j) {
+                const auto u = quat_part(tile[0][tx][il]), d = quat_part(tile[3][tx][il]);
+                stc(HQ + (size_t)b * mstrideq + (size_t)i * N + j, typename QuatOf<SO>::type{u.x, -u.y, -d.x, -d.y});
+            }
+            continue;
+        }
         if (i < N && j < N && i >= j) {
             put(j, i + N, conj_stored(tile[2][tx][il]));  // UD(j, i) = conj DU(i, j)
             if (i > j) {
@@ -791,10 +823,10 @@ void launch_assemble(const DevParams& P, const cx<double>* Vloc, const double2* 
     const int    T    = (P.N + 31) / 32;
     dim3         grd(T * (T + 1) / 2, batch);
     const size_t smem = sizeof(SO) * 4 * 32 * 33;
-    auto         kern = P.nl ? k_assemble_soc_tiles<true, false, SO> : k_assemble_soc_tiles<false, false, SO>;
+    auto         kern = P.nl ? k_assemble_soc_tiles<true, false, false, SO> : k_assemble_soc_tiles<false, false, false, SO>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, H, ld, mstride, H32, mstride32, batch, DevParamsDS{}, nullptr,
-                                nullptr, nullptr, nullptr);
+                                nullptr, nullptr, nullptr, nullptr, 0);
     count_launch();
 }
 
@@ -815,19 +847,33 @@ template <typename SO>
 void launch_assemble_soc_ds(const DevParams& P, const DevParamsDS& Q, const float4* Vloc32, const float4* phNL32,
                             const float4* phSO32, const float2* rows32, const cx<double>* Vloc, const double2* phNL,
                             const double2* phSO, const double* rows, SO* H, int ld, size_t mstride,
-                            typename Lower<SO>::type* H32, size_t mstride32, int batch, cudaStream_t s) {
+                            typename Lower<SO>::type* H32, size_t mstride32, int batch, cudaStream_t s, qt<float>* HQ,
+                            size_t mstrideq) {
     const int    T    = (P.N + 31) / 32;
     dim3         grd(T * (T + 1) / 2, batch), blk(32, 8);
     const size_t smem = sizeof(SO) * 4 * 32 * 33;
-    auto         kern = P.nl ? k_assemble_soc_tiles<true, true, SO> : k_assemble_soc_tiles<false, true, SO>;
+    auto         kern = HQ ? (P.nl ? k_assemble_soc_tiles<true, true, true, SO> : k_assemble_soc_tiles<false, true, true, SO>)
+                           : (P.nl ? k_assemble_soc_tiles<true, true, false, SO> : k_assemble_soc_tiles<false, true, false, SO>);
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, H, ld, mstride, H32, mstride32, batch, Q, Vloc32, phNL32, phSO32,
-                                rows32);
+                                rows32, HQ, mstrideq);
+    count_launch();
+}
+void launch_assemble_quat(const DevParams& P, const cx<double>* Vloc, const double2* phNL, const double2* phSO,
+                          const double* rows, qt<double>* HQ, size_t mstrideq, int batch, cudaStream_t s) {
+    using SO          = cx<double>;
+    const int    T    = (P.N + 31) / 32;
+    dim3         grd(T * (T + 1) / 2, batch), blk(32, 8);
+    const size_t smem = sizeof(SO) * 4 * 32 * 33;
+    auto         kern = P.nl ? k_assemble_soc_tiles<true, false, true, SO> : k_assemble_soc_tiles<false, false, true, SO>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, nullptr, 0, 0, nullptr, 0, batch, DevParamsDS{}, nullptr, nullptr,
+                                nullptr, nullptr, HQ, mstrideq);
     count_launch();
 }
 template void launch_assemble_soc_ds<ds4>(const DevParams&, const DevParamsDS&, const float4*, const float4*, const float4*,
                                           const float2*, const cx<double>*, const double2*, const double2*, const double*,
-                                          ds4*, int, size_t, cx<float>*, size_t, int, cudaStream_t);
+                                          ds4*, int, size_t, cx<float>*, size_t, int, cudaStream_t, qt<float>*, size_t);
 
 // ---- diagnostics: the mixed path's double-single special functions on device values -----------
 __global__ void k_ds_special(int fn, const double* __restrict__ x, size_t n, double* __restrict__ y) {

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                                                                    cx<typename ST<S>::R>* __restrict__ Xout,
                                                                    const DevParams P, const double* __restrict__ kpts,
                                                                    const int* __restrict__ G, double* __restrict__ grad,
-                                                                   int batch) {
+                                                                   int batch, int nbo) {
     using R          = typename ST<S>::R;
     const int     b  = blockIdx.x;
     if (b >= batch) return;
@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                         const R* src = reinterpret_cast<const R*>(ac + r);
                         R*       dst = reinterpret_cast<R*>(vs + r);
                         cp_async_elem<sizeof(R)>(dst, src);
-                        if constexpr (sizeof(S) != sizeof(R)) cp_async_elem<sizeof(R)>(dst + 1, src + 1);
+#pragma unroll
+                        for (int q = 1; q < (int)(sizeof(S) / sizeof(R)); ++q) cp_async_elem<sizeof(R)>(dst + q, src + q);
                     } else {
                         vs[r] = (r == i + 1) ? ST<S>::one() : ST<S>::zero();
                     }
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                 const S*  vrow = Vs + (packed_off<LPV>(ihi, ldv) - off0) - LPV * tc + gl;
                 for (int i = ihi; i >= ilo; --i, vrow -= len) {
                     const S tau = taus[i];
-                    if (ST<S>::re(tau) == R(0) && ST<S>::im(tau) == R(0)) continue;  // uniform
+                    if (ST<S>::norm(tau) == R(0)) continue;  // uniform
                     S dot0 = ST<S>::zero(), dot1 = ST<S>::zero();
 #pragma unroll
                     for (int t = tc; t < T; ++t) {
@@ -129,7 +130,12 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                     S dot = cadd(dot0, dot1);
 #pragma unroll
                     for (int o = LPV / 2; o > 0; o >>= 1) {
-                        if constexpr (sizeof(S) == sizeof(R)) {
+                        if constexpr (is_quat<S>::value) {
+                            dot.w += __shfl_xor_sync(0xffffffffu, dot.w, o);
+                            dot.x += __shfl_xor_sync(0xffffffffu, dot.x, o);
+                            dot.y += __shfl_xor_sync(0xffffffffu, dot.y, o);
+                            dot.z += __shfl_xor_sync(0xffffffffu, dot.z, o);
+                        } else if constexpr (sizeof(S) == sizeof(R)) {
                             dot += __shfl_xor_sync(0xffffffffu, dot, o);
                         } else {
                             dot = ST<S>::make(ST<S>::re(dot) + __shfl_xor_sync(0xffffffffu, ST<S>::re(dot), o),
@@ -142,7 +148,24 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                 }
             }
         }
-        if (Xout && has) {
+        if constexpr (is_quat<S>::value) {
+            // a + b j, a = w + i x, b = y + i z: the spinors (a, -conj b) and (b, conj a)
+            if (Xout && has) {
+                cx<R>* xo = Xout + ((size_t)b * nbo + 2 * j) * 2 * n;
+#pragma unroll
+                for (int t = 0; t < T; ++t) {
+                    const int r = gl + LPV * t;
+                    if (r < n) {
+                        stc(xo + r, mk<R>(zr[t].w, zr[t].x));
+                        stc(xo + n + r, mk<R>(-zr[t].y, zr[t].z));
+                        if (2 * j + 1 < nbo) {
+                            stc(xo + 2 * n + r, mk<R>(zr[t].y, zr[t].z));
+                            stc(xo + 3 * n + r, mk<R>(zr[t].w, -zr[t].x));
+                        }
+                    }
+                }
+            }
+        } else if (Xout && has) {
             cx<R>* xo = Xout + ((size_t)b * nb + j) * n;
 #pragma unroll
             for (int t = 0; t < T; ++t) {
@@ -173,10 +196,15 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
                 sz += __shfl_xor_sync(0xffffffffu, sz, o);
             }
             if (has && gl == 0) {
-                double* go = grad + ((size_t)b * nb + j) * 3;
-                go[0]      = (sx * P.grad_pref) * P.frac_to_phys;
-                go[1]      = (sy * P.grad_pref) * P.frac_to_phys;
-                go[2]      = (sz * P.grad_pref) * P.frac_to_phys;
+                constexpr int M = is_quat<S>::value ? 2 : 1;  // bands per vector (a pair has one gradient)
+#pragma unroll
+                for (int q = 0; q < M; ++q) {
+                    if (M * j + q >= nbo) break;
+                    double* go = grad + ((size_t)b * nbo + M * j + q) * 3;
+                    go[0]      = (sx * P.grad_pref) * P.frac_to_phys;
+                    go[1]      = (sy * P.grad_pref) * P.frac_to_phys;
+                    go[2]      = (sz * P.grad_pref) * P.frac_to_phys;
+                }
             }
         }
     }
@@ -185,7 +213,7 @@ __global__ void __launch_bounds__(32 * kBtMaxWarps) k_backtransform(const S* __r
 template <typename S, int LPV, int T>
 static void bt_launch(const S* H, int n, int ld, size_t mstride, const S* tq, const typename ST<S>::R* z, int nb,
                       cx<typename ST<S>::R>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
-                      int batch, cudaStream_t s) {
+                      int batch, cudaStream_t s, int nbo) {
     constexpr int GW    = 32 / LPV;
     const int     warps = std::min(kBtMaxWarps, (nb + GW - 1) / GW);
     const int     ldv   = LPV * T;
@@ -194,7 +222,7 @@ static void bt_launch(const S* H, int n, int ld, size_t mstride, const S* tq, co
     const size_t  smem  = sizeof(S) * ((size_t)cap + n);
     auto          kern  = k_backtransform<S, LPV, T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<batch, 32 * warps, smem, s>>>(H, n, ld, mstride, tq, z, nb, cap, Xout, P, d_k, d_G, grad, batch);
+    kern<<<batch, 32 * warps, smem, s>>>(H, n, ld, mstride, tq, z, nb, cap, Xout, P, d_k, d_G, grad, batch, nbo);
     count_launch();
 }
 
@@ -210,7 +238,7 @@ void launch_backtransform(const S* H, int n, int ld, size_t mstride, const S* tq
     if (lanes && (n + lanes - 1) / lanes > tmax) lanes = 0;
     if (!lanes) lanes = (n + 7) / 8 <= tmax ? 8 : (n + 15) / 16 <= tmax ? 16 : 32;
     const int t = (n + lanes - 1) / lanes;
-#define UEPM_BT(L_, T_) bt_launch<S, L_, T_>(H, n, ld, mstride, tq, z, nb, Xout, P, d_k, d_G, grad, batch, s)
+#define UEPM_BT(L_, T_) bt_launch<S, L_, T_>(H, n, ld, mstride, tq, z, nb, Xout, P, d_k, d_G, grad, batch, s, nb)
     if (lanes == 8) {
         if (t <= 12) UEPM_BT(8, 12);
         else if (t <= 18) UEPM_BT(8, 18);
@@ -236,5 +264,34 @@ UEPM_BT_INST(float)
 UEPM_BT_INST(cx<double>)
 UEPM_BT_INST(cx<float>)
 #undef UEPM_BT_INST
+
+// Quaternion matrices: at most 12 quaternion rows per lane (48 register words), and orders to 256.
+template <typename T>
+void launch_backtransform_quat(const qt<T>* H, int n, int ld, size_t mstride, const qt<T>* tq, const T* z, int nz, int nb,
+                               cx<T>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
+                               int batch, cudaStream_t s) {
+#define UEPM_BTQ(L_, T_) bt_launch<qt<T>, L_, T_>(H, n, ld, mstride, tq, z, nz, Xout, P, d_k, d_G, grad, batch, s, nb)
+    if (n <= 96) UEPM_BTQ(8, 12);
+    else if (n <= 144) UEPM_BTQ(16, 9);
+    else if (n <= 192) UEPM_BTQ(16, 12);
+    else UEPM_BTQ(32, 8);
+#undef UEPM_BTQ
+}
+template void launch_backtransform_quat<float>(const qt<float>*, int, int, size_t, const qt<float>*, const float*, int, int,
+                                               cx<float>*, const DevParams&, const double*, const int*, double*, int,
+                                               cudaStream_t);
+template void launch_backtransform_quat<double>(const qt<double>*, int, int, size_t, const qt<double>*, const double*, int,
+                                                int, cx<double>*, const DevParams&, const double*, const int*, double*,
+                                                int, cudaStream_t);
+
+__global__ void k_pair_values(const double* __restrict__ ev, int nz, double* __restrict__ E, int nb, int total) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < total) E[t] = ev[(size_t)(t / nb) * nz + (t % nb) / 2];
+}
+void launch_pair_values(const double* ev, int nz, double* E, int nb, int batch, cudaStream_t s) {
+    const int total = batch * nb;
+    k_pair_values<<<(total + 255) / 256, 256, 0, s>>>(ev, nz, E, nb, total);
+    count_launch();
+}
 
 }  // namespace uepm

@@ -155,6 +155,10 @@ struct Layout {
     size_t rows, rows32, H, H32, d, e, tq, ev, work, z, X32, refine, small, total;
 };
 
+// Whether a solve reduces the quaternion form of H(k): where the matrix has it and neither the complex
+// kernels nor a reduction kernel of the complex matrix is asked for.
+bool quaternionic(const uepm_ctx* ctx) { return ctx->quat_h && !ctx->force_cx && ctx->tune.reduction == 0; }
+
 // Bytes of workspace one chunk of `c` matrices needs, with the offset of every region.
 Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
     const size_t n = ctx->n, N = ctx->N;
@@ -178,7 +182,7 @@ Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
     L.d    = take(c * n * rs);
     L.e    = take(c * n * rs);
     L.tq   = take(c * n * (mixed ? es32 : es));
-    L.ev   = mixed ? take(c * m * rs) : 0;
+    L.ev   = mixed || quaternionic(ctx) ? take(c * m * rs) : 0;
     if (mixed || vecs) {
         L.work = take(c * invit_work_elems<double>((int)n) * rs);
         L.z    = take(c * m * n * rs);
@@ -232,6 +236,42 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
         ProfScope p(ctx, s, KK_ROWS);
         launch_rows(ctx->P, kk, ctx->d_G, rows, c, s, rows32);
     }
+    const bool quat = quaternionic(ctx);
+    const int  N = ctx->N, nz = (m + 1) / 2;  // quaternion order, pairs
+    if (ctx->precision != UEPM_PREC_MIXED && quat) {
+        if constexpr (ST<S>::cplx) {
+            const size_t qs = (size_t)N * N;
+            auto*        HQ = reinterpret_cast<qt<double>*>(H);
+            auto*        d  = reinterpret_cast<double*>(ws + L.d);
+            auto*        e  = reinterpret_cast<double*>(ws + L.e);
+            auto*        tq = reinterpret_cast<qt<double>*>(ws + L.tq);
+            auto*        ev = reinterpret_cast<double*>(ws + L.ev);
+            {
+                ProfScope p(ctx, s, KK_ASSEMBLE);
+                launch_assemble_quat(ctx->P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, HQ, qs, c, s);
+            }
+            {
+                ProfScope p(ctx, s, KK_TRIDIAG64);
+                launch_tridiag_quat(HQ, N, N, qs, d, e, tq, st, c, s, ctx->tune.ctas_per_sm);
+            }
+            {
+                ProfScope p(ctx, s, KK_BISECT);
+                launch_bisect<double>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st);
+                launch_pair_values(ev, nz, E, nb, c, s);
+            }
+            if (vec) {
+                auto* work = reinterpret_cast<double*>(ws + L.work);
+                auto* z    = reinterpret_cast<double*>(ws + L.z);
+                {
+                    ProfScope p(ctx, s, KK_INVIT);
+                    launch_invit<double>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
+                }
+                ProfScope p(ctx, s, KK_BACKTRANSFORM);
+                launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, ctx->P, kk, ctx->d_G, gr, c, s);
+            }
+        }
+        return;
+    }
     if (ctx->precision != UEPM_PREC_MIXED) {
         {
             ProfScope p(ctx, s, KK_ASSEMBLE);
@@ -278,7 +318,8 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
         else if (ds_asm && ctx->ds_soc) {
             if constexpr (std::is_same<SP, ds4>::value)
                 launch_assemble_soc_ds<SP>(ctx->P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, ctx->d_phSO32, rows32, ctx->d_Vloc,
-                                           ctx->d_phNL, ctx->d_phSO, rows, Hs, n, mstride, H32, mstride, c, s);
+                                           ctx->d_phNL, ctx->d_phSO, rows, Hs, n, mstride, quat ? nullptr : H32, mstride, c,
+                                           s, quat ? reinterpret_cast<qt<float>*>(H32) : nullptr, (size_t)N * N);
         } else if (ds_asm)
             launch_assemble_ds<SP>(ctx->P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, rows32, ctx->d_Vloc, ctx->d_phNL, rows, Hs, n,
                                    mstride, H32, mstride, c, s);
@@ -294,6 +335,27 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
     auto* X32   = reinterpret_cast<cx<float>*>(ws + L.X32);
     auto* rw    = reinterpret_cast<S*>(ws + L.refine);
     auto* small = reinterpret_cast<S*>(ws + L.small);
+    if (quat) {
+        // the quaternion matrix (order N, in H32's place) has each level once: half the values and
+        // vectors, whose back-transformation gives both members of the pair
+        auto*        HQ = reinterpret_cast<qt<float>*>(H32);
+        auto*        qq = reinterpret_cast<qt<float>*>(tq);
+        const size_t qs = (size_t)N * N;
+        {
+            ProfScope p(ctx, s, KK_TRIDIAG32);
+            launch_tridiag_tri<qt<float>>(HQ, N, N, qs, d, e, qq, st, c, s);
+        }
+        {
+            ProfScope p(ctx, s, KK_BISECT);
+            launch_bisect<float>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st);
+        }
+        {
+            ProfScope p(ctx, s, KK_INVIT);
+            launch_invit<float>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
+        }
+        ProfScope p(ctx, s, KK_BACKTRANSFORM);
+        launch_backtransform_quat<float>(HQ, N, N, qs, qq, z, nz, m, X32, ctx->P, kk, ctx->d_G, nullptr, c, s);
+    } else {
     {
         ProfScope p(ctx, s, KK_TRIDIAG32);
         if constexpr (kReal32) {
@@ -319,6 +381,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
         ProfScope p(ctx, s, KK_BACKTRANSFORM);
         launch_backtransform<S32>(H32, n, n, mstride, tq, z, m, X32, ctx->P, kk, ctx->d_G, nullptr, c, s,
                                   ctx->tune.vector_lanes);
+    }
     }
     {
         ProfScope p(ctx, s, KK_REFINE_PROJECT);
@@ -490,6 +553,11 @@ int uepm_ctx_create(const uepm_material* mat, const int32_t* G, int N, uint32_t 
                                  mat->R2_anion == mat->R2_cation);
     ctx->real_h = !soc && mat->V3A == 0.0 && mat->V4A == 0.0 && mat->V8A == 0.0 && mat->V11A == 0.0 && same_nl;
     ctx->real   = ctx->real_h;
+    // Quaternionic: the spin-orbit phase has no antisymmetric part (lambda_1 = lambda_2, or no spin-orbit
+    // strength), as the scalar part has none. The functional needs 2 N <= 512.
+    ctx->quat_h = soc && mat->V3A == 0.0 && mat->V4A == 0.0 && mat->V8A == 0.0 && mat->V11A == 0.0 && same_nl &&
+                  (mat->mu_soc == 0.0 || (mat->period_anion == mat->period_cation && mat->alpha_soc == 1.0 &&
+                                          mat->radial_extent_anion == mat->radial_extent_cation));
     cudaGetDevice(&ctx->device);
 
     // Derived constants, each with the reference's own expression.

@@ -20,6 +20,9 @@ struct uepm_ctx {
     bool          real_h    = false;  // H(k) is exactly real for this material and flags
     bool          force_cx  = false;  // run the complex kernels even when H(k) is real
     bool          real      = false;  // real_h && !force_cx
+    // H(k) of a spin-orbit context is quaternionic: time reversal times inversion is a symmetry at every
+    // k (no antisymmetric form factors, equal atoms), so every level is a Kramers pair
+    bool          quat_h    = false;
     size_t        ws_limit  = (size_t)8 << 30;
     uepm_tuning   tune{};  // kernel-shape choices (0: automatic)
     int*          d_G       = nullptr;

@@ -41,7 +41,7 @@ constexpr int kUpd = 4;  // elements per thread per round of the rank-2 update
 // fewer for complex FP64 with many row chunks (whose accumulators alone take 4 MAXT registers).
 template <typename S, int MAXT>
 constexpr int tridiag_min_blocks() {
-    return sizeof(S) * MAXT <= 8 * 5 ? 5 : (sizeof(S) <= 8 || MAXT <= 5 ? 4 : (MAXT <= 8 ? 3 : 2));
+    return is_quat<S>::value ? 2 : sizeof(S) * MAXT <= 8 * 5 ? 5 : (sizeof(S) <= 8 || MAXT <= 5 ? 4 : (MAXT <= 8 ? 3 : 2));
 }
 
 template <typename S, int NT, int MAXT, bool SMEM>
@@ -93,7 +93,9 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
             const R c0r = ST<S>::re(c0), c0i = ST<S>::im(c0);
             R       beta;
             S       th, sc;
-            if (tail2 <= num<R>::tiny() && c0i * c0i <= num<R>::tiny()) {
+            if constexpr (is_quat<S>::value) {
+                quat_reflector(c0, tail2, num<R>::tiny(), beta, th, sc);
+            } else if (tail2 <= num<R>::tiny() && c0i * c0i <= num<R>::tiny()) {
                 th   = ST<S>::zero();
                 sc   = ST<S>::zero();
                 beta = c0r;
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
             }
             s_th   = th;
             s_sc   = sc;
-            s_skip = (ST<S>::re(th) == R(0) && ST<S>::im(th) == R(0));
+            s_skip = ST<S>::norm(th) == R(0);
             const R di = ST<S>::re(A[(size_t)i * ld + i]);
             dOut[(size_t)b * n + i]  = di;
             eOut[(size_t)b * n + i]  = beta;
@@ -179,11 +181,17 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
             S p = pacc[r];
 #pragma unroll
             for (int q = 1; q < NW; ++q) p = cadd(p, pacc[q * n + r]);
-            const S wr = cmul(th, p);
-            w[r]       = wr;
-            part2      = cfmac(wr, v[r], part2);
+            if constexpr (is_quat<S>::value) {  // w = p tau, and Re(v^H p)
+                w[r] = cmul(p, th);
+                part2.w += re_dot(v[r], p);
+            } else {
+                const S wr = cmul(th, p);
+                w[r]       = wr;
+                part2      = cfmac(wr, v[r], part2);
+            }
         }
-        part2 = warp_sum(part2);
+        if constexpr (is_quat<S>::value) part2.w = warp_sum(part2.w);
+        else part2 = warp_sum(part2);
         if (lane == 0) {
             red[NW + warp]     = ST<S>::re(part2);
             red[2 * NW + warp] = ST<S>::im(part2);
@@ -195,8 +203,13 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
             wvr += red[NW + q];
             wvi += red[2 * NW + q];
         }
-        const S alpha = cscale(cmul(th, ST<S>::make(wvr, wvi)), R(-0.5));
-        for (int r = tid; r < m; r += NT) w[r] = cfma(alpha, v[r], w[r]);
+        if constexpr (is_quat<S>::value) {  // v^H A v is real: -|tau|^2 (v^H p) / 2
+            const R g = R(-0.5) * wvr * ST<S>::norm(th);
+            for (int r = tid; r < m; r += NT) w[r] = cadd(w[r], cscale(v[r], g));
+        } else {
+            const S alpha = cscale(cmul(th, ST<S>::make(wvr, wvi)), R(-0.5));
+            for (int r = tid; r < m; r += NT) w[r] = cfma(alpha, v[r], w[r]);
+        }
         __syncthreads();
 
         // ---- A22 -= v w^H + w v^H: lower triangle computed, upper mirrored -------------------
@@ -765,6 +778,14 @@ static void tridiag_pick(S* H, int n, int ld, size_t mstride, typename ST<S>::R*
                          int* status, int batch, cudaStream_t s, int ctas_per_sm) {
     if (use_smem<S>(n)) tridiag_launch_t<S, 256, MAXT, true>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
     else tridiag_launch_t<S, 256, MAXT, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
+}
+
+void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d, double* e, qt<double>* tq, int* status,
+                         int batch, cudaStream_t s, int ctas_per_sm) {
+    using S = qt<double>;
+    if (n <= 128) tridiag_launch_t<S, 256, 4, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
+    else if (n <= 192) tridiag_launch_t<S, 256, 6, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
+    else tridiag_launch_t<S, 256, 8, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
 }
 
 template <typename S>

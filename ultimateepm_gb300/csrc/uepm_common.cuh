@@ -56,6 +56,74 @@ __device__ __forceinline__ cx<T> cscale(cx<T> a, T s) {
     return mk(a.x * s, a.y * s);
 }
 
+// Quaternions w + x i + y j + z k, for Hermitian matrices that time reversal times inversion makes
+// quaternionic (spin-orbit on an inversion-symmetric crystal): half the order of the complex spinor
+// matrix, with a quarter of its elements. The products keep the operands' order.
+template <typename T>
+struct __align__(4 * sizeof(T) <= 16 ? 4 * sizeof(T) : 16) qt {
+    T w, x, y, z;
+};
+template <typename T>
+__host__ __device__ __forceinline__ qt<T> mkq(T w, T x, T y, T z) {
+    qt<T> r;
+    r.w = w;
+    r.x = x;
+    r.y = y;
+    r.z = z;
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ qt<T> cadd(qt<T> a, qt<T> b) {
+    return mkq(a.w + b.w, a.x + b.x, a.y + b.y, a.z + b.z);
+}
+template <typename T>
+__device__ __forceinline__ qt<T> csub(qt<T> a, qt<T> b) {
+    return mkq(a.w - b.w, a.x - b.x, a.y - b.y, a.z - b.z);
+}
+template <typename T>
+__device__ __forceinline__ qt<T> cscale(qt<T> a, T s) {
+    return mkq(a.w * s, a.x * s, a.y * s, a.z * s);
+}
+// c + a * b
+template <typename T>
+__device__ __forceinline__ qt<T> cfma(qt<T> a, qt<T> b, qt<T> c) {
+    return mkq(fma(a.w, b.w, fma(-a.x, b.x, fma(-a.y, b.y, fma(-a.z, b.z, c.w)))),
+               fma(a.w, b.x, fma(a.x, b.w, fma(a.y, b.z, fma(-a.z, b.y, c.x)))),
+               fma(a.w, b.y, fma(-a.x, b.z, fma(a.y, b.w, fma(a.z, b.x, c.y)))),
+               fma(a.w, b.z, fma(a.x, b.y, fma(-a.y, b.x, fma(a.z, b.w, c.z)))));
+}
+template <typename T>
+__device__ __forceinline__ qt<T> cmul(qt<T> a, qt<T> b) {
+    return cfma(a, b, mkq<T>(0, 0, 0, 0));
+}
+// c + conj(a) * b
+template <typename T>
+__device__ __forceinline__ qt<T> cfmac(qt<T> a, qt<T> b, qt<T> c) {
+    return cfma(mkq(a.w, -a.x, -a.y, -a.z), b, c);
+}
+// c - a * conj(b)
+template <typename T>
+__device__ __forceinline__ qt<T> cfms_conjb(qt<T> a, qt<T> b, qt<T> c) {
+    return cfma(a, mkq(-b.w, b.x, b.y, b.z), c);
+}
+__device__ __forceinline__ qt<float> ldc(const qt<float>* p) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    return mkq(v.x, v.y, v.z, v.w);
+}
+__device__ __forceinline__ void stc(qt<float>* p, qt<float> a) {
+    *reinterpret_cast<float4*>(p) = make_float4(a.w, a.x, a.y, a.z);
+}
+__device__ __forceinline__ qt<double> ldc(const qt<double>* p) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2  a = q[0], b = q[1];
+    return mkq(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void stc(qt<double>* p, qt<double> a) {
+    double2* q = reinterpret_cast<double2*>(p);
+    q[0]       = make_double2(a.w, a.x);
+    q[1]       = make_double2(a.y, a.z);
+}
+
 // 16-byte (double) / 8-byte (float) vector loads and stores of one complex element.
 __device__ __forceinline__ cx<double> ldc(const cx<double>* p) {
     double2 v = *reinterpret_cast<const double2*>(p);
@@ -131,6 +199,59 @@ struct ST<cx<T>> {
     static __device__ __forceinline__ T norm(cx<T> a) { return fma(a.x, a.x, a.y * a.y); }
     static __device__ __forceinline__ cx<T> neg(cx<T> a) { return mk<T>(-a.x, -a.y); }
 };
+
+template <typename T>
+struct ST<qt<T>> {
+    using R = T;
+    static constexpr bool cplx = false;
+    static __device__ __forceinline__ qt<T> zero() { return mkq<T>(0, 0, 0, 0); }
+    static __device__ __forceinline__ qt<T> one() { return mkq<T>(1, 0, 0, 0); }
+    static __device__ __forceinline__ T re(qt<T> a) { return a.w; }
+    static __device__ __forceinline__ T im(qt<T>) { return 0; }  // of real values only
+    static __device__ __forceinline__ qt<T> make(T r, T) { return mkq<T>(r, 0, 0, 0); }
+    static __device__ __forceinline__ qt<T> conj(qt<T> a) { return mkq<T>(a.w, -a.x, -a.y, -a.z); }
+    static __device__ __forceinline__ T norm(qt<T> a) { return fma(a.w, a.w, fma(a.x, a.x, fma(a.y, a.y, a.z * a.z))); }
+    static __device__ __forceinline__ qt<T> neg(qt<T> a) { return mkq<T>(-a.w, -a.x, -a.y, -a.z); }
+};
+// The imaginary part's norm, and a scalar from a real number, for every scalar type.
+__device__ __forceinline__ float  imag_norm(float) { return 0.f; }
+__device__ __forceinline__ double imag_norm(double) { return 0.0; }
+template <typename T>
+__device__ __forceinline__ T imag_norm(cx<T> a) {
+    return a.y * a.y;
+}
+template <typename T>
+__device__ __forceinline__ T imag_norm(qt<T> a) {
+    return fma(a.x, a.x, fma(a.y, a.y, a.z * a.z));
+}
+
+template <typename S>
+struct is_quat {
+    static constexpr bool value = false;
+};
+template <typename T>
+struct is_quat<qt<T>> {
+    static constexpr bool value = true;
+};
+// Re(conj(a) b)
+template <typename T>
+__device__ __forceinline__ T re_dot(qt<T> a, qt<T> b) {
+    return fma(a.w, b.w, fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)));
+}
+// The reflector of a quaternion column (alpha; tail), |tail|^2 = tail2: H = I - v tau v^H with beta real,
+// tau = (beta - alpha) / beta and v = (1; tail sc), sc = (alpha - beta)^-1 (zlarfg's, the operands in order).
+template <typename T>
+__device__ __forceinline__ void quat_reflector(qt<T> alpha, T tail2, T tiny, T& beta, qt<T>& tau, qt<T>& sc) {
+    const T im = imag_norm(alpha);
+    beta = alpha.w;
+    tau = sc = mkq<T>(0, 0, 0, 0);
+    if (tail2 <= tiny && im <= tiny) return;
+    beta = sqrt(fma(alpha.w, alpha.w, tail2 + im));
+    if (alpha.w >= 0) beta = -beta;
+    const qt<T> df = mkq(alpha.w - beta, alpha.x, alpha.y, alpha.z);
+    tau            = cscale(df, T(-1) / beta);
+    sc             = cscale(mkq(df.w, -df.x, -df.y, -df.z), T(1) / ST<qt<T>>::norm(df));
+}
 
 // Lower-precision counterpart of a scalar type (FP64 -> FP32), for the mixed path.
 template <typename S>

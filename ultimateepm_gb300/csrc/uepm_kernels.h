@@ -24,7 +24,11 @@ template <typename SO>
 void launch_assemble_soc_ds(const DevParams& P, const DevParamsDS& Q, const float4* Vloc32, const float4* phNL32,
                             const float4* phSO32, const float2* rows32, const cx<double>* Vloc, const double2* phNL,
                             const double2* phSO, const double* rows, SO* H, int ld, size_t mstride,
-                            typename Lower<SO>::type* H32, size_t mstride32, int batch, cudaStream_t s);
+                            typename Lower<SO>::type* H32, size_t mstride32, int batch, cudaStream_t s,
+                            qt<float>* HQ = nullptr, size_t mstrideq = 0);
+// Quaternionic H (order N): HQ above receives its FP32 lower triangle; this forms the full FP64 matrix.
+void launch_assemble_quat(const DevParams& P, const cx<double>* Vloc, const double2* phNL, const double2* phSO,
+                          const double* rows, qt<double>* HQ, size_t mstrideq, int batch, cudaStream_t s);
 template <typename SO>
 void launch_assemble_ds(const DevParams& P, const DevParamsDS& Q, const float4* Vloc32, const float4* phNL32,
                         const float2* rows32, const cx<double>* Vloc, const double2* phNL, const double* rows, SO* H,
@@ -50,6 +54,9 @@ template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant = 0, int ctas_per_sm = 0, int cluster = 0,
                     bool tensor_cores = true);
+// The FP64 reduction of quaternion matrices (order n <= 256; tridiag.cu).
+void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d, double* e, qt<double>* tq, int* status,
+                         int batch, cudaStream_t s, int ctas_per_sm);
 // tridiag_cluster.cu: cluster size for order n (want = 0: automatic; 0 returned when it cannot fit)
 // and the launch (false when the cluster kernel cannot run this case).
 template <typename S>
@@ -63,6 +70,11 @@ int tridiag_blocked_max_n();
 template <typename S>
 bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq,
                             int* status, int batch, cudaStream_t s, bool tensor_cores);
+// tridiag_tri.cu: the reduction of quaternion matrices (order 1..256, H: the lower triangle, column-major)
+// with the triangle in shared memory (false when it cannot run).
+template <typename S>
+bool launch_tridiag_tri(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, int* status, int batch,
+                        cudaStream_t s);
 // tridiag_reg.cu: the same reduction for real FP32 matrices with n <= tridiag_reg_max_n(), held in
 // registers (launch_tridiag<float> dispatches to it).
 int  tridiag_reg_max_n();
@@ -94,6 +106,16 @@ template <typename S>
 void launch_backtransform(const S* H, int n, int ld, size_t mstride, const S* tq, const typename ST<S>::R* z, int nb,
                           cx<typename ST<S>::R>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
                           int batch, cudaStream_t s, int lanes = 0);
+
+// The same for a quaternion matrix of order n = N from nz real vectors z ([batch][nz][N]): quaternion
+// vector a + b j gives the spinor eigenvectors (a, -conj b) and (b, conj a), written as vectors 2 q and
+// 2 q + 1 of [batch][nb][2 N] (nb = 2 nz or 2 nz - 1), with their gradients.
+template <typename T>
+void launch_backtransform_quat(const qt<T>* H, int n, int ld, size_t mstride, const qt<T>* tq, const T* z, int nz, int nb,
+                               cx<T>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
+                               int batch, cudaStream_t s);
+// E[b][i] = ev[b][i / 2], i < nb: the doubly degenerate values of a quaternion matrix (backtransform.cu)
+void launch_pair_values(const double* ev, int nz, double* E, int nb, int batch, cudaStream_t s);
 
 // refine.cu: FP64 Rayleigh-Ritz in the m-dimensional subspace of FP32 vectors X32 ([batch][m][n]);
 // the nb lowest Ritz values go to Eout, optionally vectors / gradients.
