@@ -44,6 +44,117 @@ constexpr int tridiag_min_blocks() {
     return is_quat<S>::value ? 2 : sizeof(S) * MAXT <= 8 * 5 ? 5 : (sizeof(S) <= 8 || MAXT <= 5 ? 4 : (MAXT <= 8 ? 3 : 2));
 }
 
+template <typename T>
+__device__ __forceinline__ T shfl_xor(T a, int o) {
+    return __shfl_xor_sync(0xffffffffu, a, o);
+}
+template <typename T>
+__device__ __forceinline__ cx<T> shfl_xor(cx<T> a, int o) {
+    return mk(shfl_xor(a.x, o), shfl_xor(a.y, o));
+}
+template <typename T>
+__device__ __forceinline__ qt<T> shfl_xor(qt<T> a, int o) {
+    return mkq(shfl_xor(a.w, o), shfl_xor(a.x, o), shfl_xor(a.y, o), shfl_xor(a.z, o));
+}
+
+// zlarfg's scalars of the column (c0; tail), tail2 = |tail|^2: beta real, th = (beta - c0) / beta,
+// sc = 1 / (c0 - beta). One division serves both reciprocals (an FP64 division costs as much of the
+// FP64 pipe as a 30-row column of the product) while the products stay well inside the exponent range.
+template <typename S>
+__device__ __forceinline__ void reflector_scalars(S c0, typename ST<S>::R tail2, typename ST<S>::R& beta, S& th, S& sc) {
+    using R = typename ST<S>::R;
+    if constexpr (is_quat<S>::value) {
+        quat_reflector(c0, tail2, num<R>::tiny(), beta, th, sc);
+    } else {
+        const R c0r = ST<S>::re(c0), c0i = ST<S>::im(c0);
+        if (tail2 <= num<R>::tiny() && c0i * c0i <= num<R>::tiny()) {
+            th   = ST<S>::zero();
+            sc   = ST<S>::zero();
+            beta = c0r;
+            return;
+        }
+        beta = sqrt(fma(c0r, c0r, fma(c0i, c0i, tail2)));
+        if (c0r >= 0) beta = -beta;
+        const R ar = c0r - beta, q = fma(ar, ar, c0i * c0i);
+        R       ib, den;
+        const float mag = fabsf((float)beta);
+        if (sizeof(R) == 8 && mag > 1e-30f && mag < 1e30f) {
+            const R inv = R(1) / (beta * q);
+            ib          = inv * q;
+            den         = inv * beta;
+        } else {
+            ib  = R(1) / beta;
+            den = R(1) / q;
+        }
+        th = ST<S>::make((beta - c0r) * ib, -c0i * ib);
+        sc = ST<S>::make(ar * den, -c0i * den);
+    }
+}
+
+// pw[r] = this warp's part of (A v)_r over its columns (c = warp mod NW), A full, m x m: lanes own rows.
+// TF full 32-row chunks; the remaining rows take one instruction for 1, 2 or 4 columns (a lane group of
+// 32, 16 or 8 lanes each). The chunk count is a template parameter, so that no dead chunk is issued:
+// predicated off they still took the FP64 pipe (91 k instructions per matrix at n = 137, 70 k so).
+template <typename S, int NW, int TF>
+__device__ __forceinline__ void product_t(const S* __restrict__ A, int ld, int m, const S* v, S* pw, int warp, int lane) {
+    if constexpr (TF > 0) {
+        S acc[TF];
+#pragma unroll
+        for (int t = 0; t < TF; ++t) acc[t] = ST<S>::zero();
+        const int tf = m >> 5;
+        for (int c = warp; c < m; c += NW) {
+            const S* ac = A + (size_t)c * ld + lane;
+            const S  vc = v[c];
+            S        a[TF];
+#pragma unroll
+            for (int t = 0; t < TF; ++t) a[t] = TF <= 8 || t < tf ? ldc(ac + 32 * t) : ST<S>::zero();
+#pragma unroll
+            for (int t = 0; t < TF; ++t) acc[t] = cfma(a[t], vc, acc[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < TF; ++t)
+            if (TF <= 8 || t < tf) pw[lane + 32 * t] = acc[t];
+    }
+    const int rem = m & 31;
+    if (rem) {
+        const int lg = rem <= 8 ? 3 : rem <= 16 ? 4 : 5, g = 32 >> lg;  // 2^lg lanes per column
+        const int sub = lane >> lg, rr = (m & ~31) + (lane & ((1 << lg) - 1));
+        const S*  ar = A + rr;
+        S         at = ST<S>::zero();
+        int       c0 = warp * g;
+        for (; c0 + 3 * NW * g + g <= m; c0 += 4 * NW * g) {
+            S a[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[q] = rr < m ? ldc(ar + (size_t)(c0 + q * NW * g + sub) * ld) : ST<S>::zero();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) at = cfma(a[q], v[c0 + q * NW * g + sub], at);
+        }
+        for (; c0 < m; c0 += NW * g) {
+            const int c = c0 + sub;
+            if (c0 + g <= m || c < m) at = cfma(rr < m ? ldc(ar + (size_t)c * ld) : ST<S>::zero(), v[c], at);
+        }
+        for (int q = 16; q >= (1 << lg); q >>= 1) at = cadd(at, shfl_xor(at, q));
+        if (sub == 0 && rr < m) pw[rr] = at;
+    }
+}
+template <typename S, int NW, int MAXT>
+__device__ __forceinline__ void product(const S* A, int ld, int m, const S* v, S* pw, int warp, int lane) {
+    switch (m >> 5) {
+        case 0: product_t<S, NW, 0>(A, ld, m, v, pw, warp, lane); break;
+        case 1: product_t<S, NW, 1>(A, ld, m, v, pw, warp, lane); break;
+        case 2: product_t<S, NW, 2>(A, ld, m, v, pw, warp, lane); break;
+        case 3: product_t<S, NW, 3>(A, ld, m, v, pw, warp, lane); break;
+        case 4: if constexpr (MAXT >= 4) product_t<S, NW, 4>(A, ld, m, v, pw, warp, lane); break;
+        case 5: if constexpr (MAXT >= 5) product_t<S, NW, 5>(A, ld, m, v, pw, warp, lane); break;
+        case 6: if constexpr (MAXT >= 6) product_t<S, NW, 6>(A, ld, m, v, pw, warp, lane); break;
+        case 7: if constexpr (MAXT >= 7) product_t<S, NW, 7>(A, ld, m, v, pw, warp, lane); break;
+        case 8: if constexpr (MAXT >= 8) product_t<S, NW, 8>(A, ld, m, v, pw, warp, lane); break;
+        case 9: case 10: case 11:
+        case 12: if constexpr (MAXT >= 12) product_t<S, NW, 12>(A, ld, m, v, pw, warp, lane); break;
+        default: if constexpr (MAXT >= 16) product_t<S, NW, 16>(A, ld, m, v, pw, warp, lane); break;
+    }
+}
+
 template <typename S, int NT, int MAXT, bool SMEM>
 __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) k_tridiag(S* __restrict__ H, int n, int ldg, size_t mstride,
                                                 typename ST<S>::R* __restrict__ dOut, typename ST<S>::R* __restrict__ eOut,
@@ -56,8 +167,8 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
     S*        v    = SMEM ? As + (size_t)n * lds : As;  // n
     S*        w    = v + n;                        // n
     S*        pacc = w + n;                        // NW * n
-    R*        red  = reinterpret_cast<R*>(pacc + NW * n);  // 3 * NW
-    __shared__ S   s_th, s_sc;
+    __shared__ S   s_th, s_sc, red2[NW];
+    __shared__ R   red[NW];
     __shared__ int s_skip;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // The grid may be smaller than the batch: each CTA reduces matrices b, b + gridDim.x, ... so the
@@ -75,140 +186,119 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
         __syncthreads();
     }
 
+    // xc: this thread's rows (tid, tid + NT) of the column to reduce next, and ss their norm's sum over
+    // the tail; from the matrix for column 0, from the previous column's update afterwards
+    S xc[2];
+    R ss = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int r = tid + k * NT;  // row o + r - 1 of column 0: r = 0 is the diagonal
+        xc[k]       = r < n ? ldc(A + r) : ST<S>::zero();
+        if (r >= 2 && r < n) ss += ST<S>::norm(xc[k]);
+    }
     for (int i = 0; i < n - 1; ++i) {
         const int o = i + 1, m = n - o;
         S*        col = A + (size_t)i * ld + o;
 
         // ---- Householder vector of A[o:, i] -------------------------------------------------
-        R part = 0;
-        for (int r = 1 + tid; r < m; r += NT) part += ST<S>::norm(ldc(col + r));
-        part = warp_sum(part);
-        if (lane == 0) red[warp] = part;
+        // The column's rows are in the registers of the threads that updated it (thread r: row i + r),
+        // so nothing is read back, and each warp that holds some sums its squares.
+        if (32 * warp <= m) {
+            ss = warp_sum(ss);
+            if (lane == 0) red[warp] = ss;
+        }
+        if (tid == 1) s_sc = xc[0];  // c0
         __syncthreads();
-        if (tid == 0) {
-            R tail2 = 0;
-#pragma unroll
-            for (int q = 0; q < NW; ++q) tail2 += red[q];
-            const S c0 = ldc(col);
-            const R c0r = ST<S>::re(c0), c0i = ST<S>::im(c0);
-            R       beta;
-            S       th, sc;
-            if constexpr (is_quat<S>::value) {
-                quat_reflector(c0, tail2, num<R>::tiny(), beta, th, sc);
-            } else if (tail2 <= num<R>::tiny() && c0i * c0i <= num<R>::tiny()) {
-                th   = ST<S>::zero();
-                sc   = ST<S>::zero();
-                beta = c0r;
-            } else {
-                beta = sqrt(fma(c0r, c0r, fma(c0i, c0i, tail2)));
-                if (c0r >= 0) beta = -beta;
-                const R ib = R(1) / beta;
-                th         = ST<S>::make((beta - c0r) * ib, -c0i * ib);
-                // sc = 1 / (c0 - beta)
-                const R ar = c0r - beta, ai = c0i;
-                const R den = R(1) / fma(ar, ar, ai * ai);
-                sc          = ST<S>::make(ar * den, -ai * den);
+        if (warp == 0) {
+            R tail2 = red[0];
+            for (int q = 1; q < NW && 32 * q <= m; ++q) tail2 += red[q];
+            R beta;
+            S th, sc;
+            reflector_scalars(s_sc, tail2, beta, th, sc);
+            __syncwarp();
+            if (lane == 0) {
+                const R di = ST<S>::re(xc[0]);
+                s_th   = th;
+                s_sc   = sc;
+                s_skip = ST<S>::norm(th) == R(0);
+                dOut[(size_t)b * n + i]  = di;
+                eOut[(size_t)b * n + i]  = beta;
+                tqOut[(size_t)b * n + i] = th;
+                stc(col, ST<S>::make(beta, R(0)));
+                if (!isfinite(beta) || !isfinite(di)) bad = true;
             }
-            s_th   = th;
-            s_sc   = sc;
-            s_skip = ST<S>::norm(th) == R(0);
-            const R di = ST<S>::re(A[(size_t)i * ld + i]);
-            dOut[(size_t)b * n + i]  = di;
-            eOut[(size_t)b * n + i]  = beta;
-            tqOut[(size_t)b * n + i] = th;
-            stc(col, ST<S>::make(beta, R(0)));
-            if (!isfinite(beta) || !isfinite(di)) bad = true;
         }
         __syncthreads();
         const S th = s_th, sc = s_sc;
-        for (int r = tid; r < m; r += NT) {
-            S vr;
-            if (r == 0) {
-                vr = ST<S>::one();
-            } else {
-                vr = cmul(ldc(col + r), sc);
-                stc(col + r, vr);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int r = tid + k * NT - 1;
+            if (r >= 0 && r < m) {
+                const S vr = r == 0 ? ST<S>::one() : cmul(xc[k], sc);
+                v[r]       = vr;
+                if (r > 0) stc(col + r, vr);
             }
-            v[r] = vr;
         }
         __syncthreads();
-        if (s_skip) continue;
+        ss = 0;
+        if (s_skip) {  // the next column as it stands
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int r = tid + k * NT;
+                xc[k]       = r < m ? ldc(A + (size_t)o * ld + o + r) : ST<S>::zero();
+                if (r >= 2 && r < m) ss += ST<S>::norm(xc[k]);
+            }
+            __syncthreads();
+            continue;
+        }
 
         // ---- p = A22 v (full storage): warps own columns, lanes own rows ----------------------
-        S acc[MAXT];
-#pragma unroll
-        for (int t = 0; t < MAXT; ++t) acc[t] = ST<S>::zero();
-        const int tn = (m + 31) >> 5;
-        // FP32 matrices beyond the on-chip sizes reduce from L2/DRAM and wait on memory: there the
-        // column's chunks are all loaded before the first FMA (Ge SOC n = 362: 242 -> 220 ms per
-        // 2000 k). The FP64 kernel is FP64-pipe bound and keeps the interleaved form (11.2 vs
-        // 12.0 ms at n = 137), as do the shapes where the extra registers would spill.
-        constexpr bool kBatchLoads = sizeof(R) == 4 && MAXT <= 12;
-        for (int c = warp; c < m; c += NW) {
-            const S* ac = A + (size_t)(o + c) * ld + o;
-            const S  vc = v[c];
-            if constexpr (kBatchLoads) {
-                S a[MAXT];
-#pragma unroll
-                for (int t = 0; t < MAXT; ++t) {
-                    const int r = lane + 32 * t;
-                    a[t]        = (t < tn && r < m) ? ldc(ac + r) : ST<S>::zero();
-                }
-#pragma unroll
-                for (int t = 0; t < MAXT; ++t)
-                    if (t < tn) acc[t] = cfma(a[t], vc, acc[t]);  // warp-uniform
-            } else {
-#pragma unroll
-                for (int t = 0; t < MAXT; ++t) {
-                    if (t < tn) {  // warp-uniform
-                        const int r = lane + 32 * t;
-                        const S   a = (r < m) ? ldc(ac + r) : ST<S>::zero();
-                        acc[t]      = cfma(a, vc, acc[t]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < MAXT; ++t) {
-            const int r = lane + 32 * t;
-            if (t < tn && r < m) pacc[warp * n + r] = acc[t];
-        }
+        product<S, NW, MAXT>(A + (size_t)o * ld + o, ld, m, v, pacc + warp * n, warp, lane);
         __syncthreads();
 
         // ---- w = tau p; alpha = -tau/2 (w^H v) -------------------------------------------------
-        S part2 = ST<S>::zero();
-        for (int r = tid; r < m; r += NT) {
-            S p = pacc[r];
+        S wr[2], part2 = ST<S>::zero();
 #pragma unroll
-            for (int q = 1; q < NW; ++q) p = cadd(p, pacc[q * n + r]);
-            if constexpr (is_quat<S>::value) {  // w = p tau, and Re(v^H p)
-                w[r] = cmul(p, th);
-                part2.w += re_dot(v[r], p);
-            } else {
-                const S wr = cmul(th, p);
-                w[r]       = wr;
-                part2      = cfmac(wr, v[r], part2);
+        for (int k = 0; k < 2; ++k) {
+            const int r = tid + k * NT;
+            wr[k]       = ST<S>::zero();
+            if (r < m) {
+                S p = pacc[r];
+#pragma unroll
+                for (int q = 1; q < NW; ++q) p = cadd(p, pacc[q * n + r]);
+                if constexpr (is_quat<S>::value) {  // w = p tau, and Re(v^H p)
+                    wr[k] = cmul(p, th);
+                    part2.w += re_dot(v[r], p);
+                } else {
+                    wr[k] = cmul(th, p);
+                    part2 = cfmac(wr[k], v[r], part2);
+                }
             }
         }
-        if constexpr (is_quat<S>::value) part2.w = warp_sum(part2.w);
-        else part2 = warp_sum(part2);
-        if (lane == 0) {
-            red[NW + warp]     = ST<S>::re(part2);
-            red[2 * NW + warp] = ST<S>::im(part2);
+        if (32 * warp < m) {
+            if constexpr (ST<S>::cplx) {
+                part2 = warp_sum(part2);
+            } else {
+                part2 = ST<S>::make(warp_sum(ST<S>::re(part2)), R(0));
+            }
+            if (lane == 0) red2[warp] = part2;
         }
         __syncthreads();
-        R wvr = 0, wvi = 0;
+        if (32 * warp < m) {
+            S wv = red2[0];
+            for (int q = 1; q < NW && 32 * q < m; ++q) {
+                if constexpr (is_quat<S>::value) wv.w += red2[q].w;
+                else wv = cadd(wv, red2[q]);
+            }
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-            wvr += red[NW + q];
-            wvi += red[2 * NW + q];
-        }
-        if constexpr (is_quat<S>::value) {  // v^H A v is real: -|tau|^2 (v^H p) / 2
-            const R g = R(-0.5) * wvr * ST<S>::norm(th);
-            for (int r = tid; r < m; r += NT) w[r] = cadd(w[r], cscale(v[r], g));
-        } else {
-            const S alpha = cscale(cmul(th, ST<S>::make(wvr, wvi)), R(-0.5));
-            for (int r = tid; r < m; r += NT) w[r] = cfma(alpha, v[r], w[r]);
+            for (int k = 0; k < 2; ++k) {
+                const int r = tid + k * NT;
+                if (r < m) {
+                    if constexpr (is_quat<S>::value)  // v^H A v is real: -|tau|^2 (v^H p) / 2
+                        w[r] = cadd(wr[k], cscale(v[r], R(-0.5) * wv.w * ST<S>::norm(th)));
+                    else w[r] = cfma(cscale(cmul(th, wv), R(-0.5)), v[r], wr[k]);
+                }
+            }
         }
         __syncthreads();
 
@@ -218,6 +308,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
         // round has idle lanes (per-column 32-row chunks left ~16 idle lanes in every column).
         // Each thread takes its elements kUpd at a time, all loads first, so that kUpd loads per
         // thread are in flight (one at a time left every element waiting a full L2/DRAM latency).
+        // The first m elements are the next column to reduce: they stay in xc.
         {
             const int tot = m * (m + 1) / 2;
             int       c = 0, r = tid;  // (column, row) of element tid
@@ -225,6 +316,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
                 r = r - m + c + 1;
                 ++c;
             }
+            xc[0] = xc[1] = ST<S>::zero();
             for (int e0 = tid; e0 < tot; e0 += kUpd * NT) {
                 int cq[kUpd], rq[kUpd];
                 S   aq[kUpd];
@@ -253,13 +345,17 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) 
                         stc(A + (size_t)(o + rr) * ld + (o + cc), ST<S>::conj(a));
                     }
                     stc(A + (size_t)(o + cc) * ld + o + rr, a);
+                    if (q < 2 && cc == 0) {  // e0 = tid: rows tid and tid + NT of the next column
+                        xc[q] = a;
+                        if (rr >= 2) ss += ST<S>::norm(a);
+                    }
                 }
             }
         }
         __syncthreads();
     }
     if (tid == 0) {
-        const R dl = ST<S>::re(A[(size_t)(n - 1) * ld + (n - 1)]);
+        const R dl = ST<S>::re(xc[0]);
         dOut[(size_t)b * n + n - 1] = dl;
         eOut[(size_t)b * n + n - 1] = R(0);
         tqOut[(size_t)b * n + n - 1] = ST<S>::zero();
@@ -723,7 +819,7 @@ template <typename S, int NT, int MAXT, bool SMEM>
 static void tridiag_launch_t(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq,
                              int* status, int batch, cudaStream_t s, int ctas_per_sm) {
     using R           = typename ST<S>::R;
-    const size_t smem = sizeof(S) * ((SMEM ? (size_t)n * (n | 1) : 0) + (size_t)(2 + NT / 32) * n) + sizeof(R) * 3 * (NT / 32);
+    const size_t smem = sizeof(S) * ((SMEM ? (size_t)n * (n | 1) : 0) + (size_t)(2 + NT / 32) * n);
     auto         kern = k_tridiag<S, NT, MAXT, SMEM>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int grid = batch;
@@ -776,8 +872,13 @@ static bool use_smem(int n) {
 template <typename S, int MAXT>
 static void tridiag_pick(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq,
                          int* status, int batch, cudaStream_t s, int ctas_per_sm) {
-    if (use_smem<S>(n)) tridiag_launch_t<S, 256, MAXT, true>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
-    else tridiag_launch_t<S, 256, MAXT, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
+    if constexpr (sizeof(typename ST<S>::R) == 4) {
+        if (use_smem<S>(n)) {
+            tridiag_launch_t<S, 256, MAXT, true>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
+            return;
+        }
+    }
+    tridiag_launch_t<S, 256, MAXT, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
 }
 
 void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d, double* e, qt<double>* tq, int* status,
