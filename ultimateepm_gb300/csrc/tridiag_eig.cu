@@ -3,7 +3,7 @@
 // The reference computes ALL n eigenvalues with Eigen's implicit QR (Hamiltonian.cpp:125-134) and
 // then keeps the first nb (BandStructure.cpp:183-184). Here only the nb lowest are computed:
 //
-//   k_bisect  Sturm-count bisection (one warp per matrix, one lane per eigenvalue index), with
+//   k_bisect  Sturm-count bisection (1 to 32 lanes per eigenvalue index, several values per CTA), with
 //             LAPACK dstebz's pivot guard and absolute/relative stopping tolerances. Each value is
 //             the j-th smallest eigenvalue of T to about eps * ||T||.
 //   k_invit   inverse iteration (one warp per matrix, one lane per eigenvalue): LU with partial
@@ -77,8 +77,6 @@ __device__ __forceinline__ int sturm_count(const float* __restrict__ d, const fl
     return cnt;
 }
 
-// One group of LPM lanes per matrix (LPM = smallest power of two >= nb, at most 32), so a warp
-// bisects 32 / LPM matrices at once and every lane carries an eigenvalue.
 // Shared memory of one matrix in k_bisect: d and e^2 in T; for the FP64 kernel also their FP32
 // rounding (hi) and remainders (lo), for the FP32 pre-bracketing and the double-single counts.
 template <typename T>
@@ -132,31 +130,100 @@ __device__ __forceinline__ dsf ds_of(double v) {
     return dsf{h, __double2float_rn(v - (double)h)};
 }
 
+// The bisection steps of up to log2(P) levels at once, by a group of P lanes: lane gl < P - 1 counts at
+// node gl + 1 (heap order) of the tree of midpoints below [a, c], each formed as the one-lane bisection
+// forms it, and the group then walks down the tree with the counts. Every bracket, stopping test and
+// step count is the same as one lane's, so results do not depend on P; P > 1 only shortens the chain of
+// dependent Sturm counts (5 steps in the time of one for P = 32, at 31 / 5 of the work).
+// below(x): whether more than j eigenvalues lie below x. stop(a, c, mid): the phase's stopping test.
+// Returns whether the test ended it before `limit` steps.
+template <int P, typename X, typename Below, typename Stop>
+__device__ __forceinline__ bool section(X& a, X& c, int limit, int lane, Below below, Stop stop) {
+    constexpr int LV = P == 1 ? 1 : P == 4 ? 2 : P == 8 ? 3 : P == 16 ? 4 : 5;
+    const int      gl = lane & (P - 1), node = P == 1 ? 1 : gl + 1;
+    const unsigned gmask = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
+    for (int it = 0; it < limit;) {
+        X m = X(0.5) * (a + c);
+        if (stop(a, c, m)) return true;
+        if constexpr (P == 1) {
+            if (below(m)) c = m;
+            else a = m;
+            ++it;
+        } else {
+            X na = a, nc = c;
+            for (int bit = 30 - __clz(node); bit >= 0; --bit) {  // the path from the root to this lane's node
+                if ((node >> bit) & 1) na = m;
+                else nc = m;
+                m = X(0.5) * (na + nc);
+            }
+            const bool     left = gl < P - 1 && below(m);
+            const unsigned hit  = __ballot_sync(gmask, left) >> (lane & ~(P - 1));
+            int            id   = 1;
+#pragma unroll
+            for (int l = 0; l < LV; ++l) {
+                const X mid = X(0.5) * (a + c);
+                if (l > 0 && (it >= limit || stop(a, c, mid))) break;  // the loop head decides
+                const bool lf = (hit >> (id - 1)) & 1u;
+                if (lf) c = mid;
+                else a = mid;
+                id = 2 * id + (lf ? 0 : 1);
+                ++it;
+            }
+        }
+    }
+    return false;
+}
+
+// The two counts that confirm a bracket, count(lo) <= j < count(hi), by two lanes where the group has them.
+template <int P, typename Below>
+__device__ __forceinline__ bool confirm(double lo, double hi, int lane, Below below) {
+    if constexpr (P == 1) return !below(lo) && below(hi);
+    const int      gl = lane & (P - 1);
+    const unsigned gmask = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
+    const bool     mine  = gl < 2 && below(gl == 0 ? lo : hi);
+    const unsigned hit   = __ballot_sync(gmask, mine) >> (lane & ~(P - 1));
+    return (hit & 3u) == 2u;
+}
+
+struct BisectMatrix {  // what a matrix's values share
+    double lo, hi, tnorm, pivmin;
+    float  pivf;
+    int    pad;
+};
+
+// One CTA takes IPB = 128 / P values of the flattened list (matrix, j); d and e^2 of the matrices that they
+// touch are staged in shared memory. P lanes per value in the FP32 and double-single phases, Q (<= P) in
+// the last one, whose FP64 steps cost the same whatever the lane mask: there the CTA's values move
+// together into the first warps.
+//
 // Iterations per bisection phase: `cap` when positive (UEPM tuning max_iter), else 64 for the FP32
 // and double-single pre-bracketing and 200 for the final phase (which needs ~60: the range over
 // eps ||T||). An eigenvalue whose final bracket is still open when the cap ends it sets
 // UEPM_K_NOCONVERGE in status; a non-finite bracket (NaN / Inf in T) sets UEPM_K_NONFINITE.
-template <typename T>
-__global__ void k_bisect(const T* __restrict__ dIn, const T* __restrict__ eIn, int n, int nb, int lpm, T* __restrict__ evOut,
-                         int ev_ld, int batch, int cap, int* __restrict__ status) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mpw  = 32 / lpm;
-    const int g    = lane / lpm, gl = lane - g * lpm;
-    const int b    = (blockIdx.x * kBisectWarpsPerBlock + warp) * mpw + g;
+template <typename T, int P, int Q>
+__global__ void __launch_bounds__(32 * kBisectWarpsPerBlock) k_bisect(const T* __restrict__ dIn, const T* __restrict__ eIn,
+                                                                      int n, int nb, T* __restrict__ evOut, int ev_ld,
+                                                                      int batch, int cap, int* __restrict__ status) {
+    constexpr int IPB = 32 * kBisectWarpsPerBlock / P;
+    const int     tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     extern __shared__ __align__(16) unsigned char smraw[];
-    unsigned char* mine = smraw + ((size_t)warp * mpw + g) * bisect_matrix_bytes<T>(n);
-    T*             d    = reinterpret_cast<T*>(mine);
-    T*             e2   = d + n;
-    float*         df   = reinterpret_cast<float*>(e2 + n);  // FP64 kernel only: hi parts
-    float*         e2f  = df + n;
-    float*         dlo  = e2f + n;                           // lo parts
-    float*         e2lo = dlo + n;
-    const bool valid = b < batch;
-    T          lo = T(3.0e38), hi = T(-3.0e38), emax2 = T(0);
-    if (valid) {
-        const T* dg = dIn + (size_t)b * n;
-        const T* eg = eIn + (size_t)b * n;
-        for (int i = gl; i < n; i += lpm) {
+    __shared__ double s_a[IPB], s_c[IPB];
+    const long long item0 = (long long)blockIdx.x * IPB, items = (long long)batch * nb;
+    const long long last  = min(item0 + IPB, items) - 1;
+    const int       b0 = (int)(item0 / nb), nm = (int)(last / nb) - b0 + 1;  // the CTA's matrices
+    const size_t    mb    = bisect_matrix_bytes<T>(n);
+    auto*           share = reinterpret_cast<BisectMatrix*>(smraw + mb * nm);
+    for (int q = warp; q < nm; q += kBisectWarpsPerBlock) {
+        T*       d   = reinterpret_cast<T*>(smraw + mb * q);
+        T*       e2  = d + n;
+        float*   df  = reinterpret_cast<float*>(e2 + n);  // FP64 kernel only: hi parts
+        float*   e2f = df + n;
+        float*   dlo = e2f + n;                           // lo parts
+        float*   e2lo = dlo + n;
+        const T* dg  = dIn + (size_t)(b0 + q) * n;
+        const T* eg  = eIn + (size_t)(b0 + q) * n;
+        T        lo = T(3.0e38), hi = T(-3.0e38), emax2 = T(0);
+        for (int i = lane; i < n; i += 32) {
             const T di = dg[i];
             const T em = (i > 0) ? fabs(eg[i - 1]) : T(0);
             const T ep = (i < n - 1) ? fabs(eg[i]) : T(0);
@@ -176,98 +243,145 @@ __global__ void k_bisect(const T* __restrict__ dIn, const T* __restrict__ eIn, i
             lo = min(lo, di - em - ep);
             hi = max(hi, di + em + ep);
         }
+        lo    = warp_min(lo);
+        hi    = warp_max(hi);
+        emax2 = warp_max(emax2);
+        if (lane == 0) {
+            const T pivmin = num<T>::tiny() * max(T(1), emax2);
+            const T tnorm  = max(fabs(lo), fabs(hi));
+            const T widen  = T(2) * num<T>::eps() * tnorm * T(n) + T(2) * pivmin;
+            share[q]       = BisectMatrix{(double)(lo - widen), (double)(hi + widen), (double)tnorm, (double)pivmin,
+                                    FLT_MIN * fmaxf(1.f, (float)emax2), 0};
+        }
     }
-    // reductions within each lane group
-    for (int o = lpm / 2; o > 0; o >>= 1) {
-        lo    = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi    = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        emax2 = max(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
-    }
-    __syncwarp();
-    if (!valid) return;
-    const T eps    = num<T>::eps();
-    const T pivmin = num<T>::tiny() * max(T(1), emax2);
-    const T tnorm  = max(fabs(lo), fabs(hi));
-    const T widen  = T(2) * eps * tnorm * T(n) + T(2) * pivmin;
-    lo -= widen;
-    hi += widen;
-    const T   atol    = eps * tnorm;
+    __syncthreads();
+    const T   eps     = num<T>::eps();
     const int it_pre  = cap > 0 ? min(cap, 64) : 64;
     const int it_last = cap > 0 ? cap : 200;
-    int       flags   = 0;
-    for (int j = gl; j < nb; j += lpm) {
-        T a = lo, c = hi;
-        if (sizeof(T) == 8) {
-            // FP32 pre-bracketing: bisect in FP32 (the FP32 pipe is 64x wider on GB300) to ~1e-6
-            // relative, widen by 16 eps32 ||T|| (the backward error of an FP32 Sturm count is a few
-            // eps32 ||T||) and keep the bracket only if two FP64 counts confirm it.
-            const float pivf = FLT_MIN * fmaxf(1.f, (float)emax2);
-            const float tolf = 4.f * FLT_EPSILON * (float)tnorm;
-            float       af = (float)a, cf = (float)c;
-            for (int it = 0; it < it_pre; ++it) {
-                const float mf = 0.5f * (af + cf);
-                if (cf - af <= tolf || mf <= af || mf >= cf) break;
-                if (sturm_count(df, e2f, n, mf, pivf) > j) cf = mf;
-                else af = mf;
-            }
-            const T w   = T(16) * T(FLT_EPSILON) * tnorm;
-            const T lo2 = max(a, T(af) - w), hi2 = min(c, T(cf) + w);
-            if (lo2 < hi2 && sturm_count(d, e2, n, lo2, pivmin) <= j && sturm_count(d, e2, n, hi2, pivmin) > j) {
+    double    a0 = 0, c0 = 0;
+    if (sizeof(T) == 8) {
+        // groups past the end repeat the last value: whole warps stay together, and nothing is stored for them
+        const int       x    = tid / P;
+        const long long item = min(item0 + x, last);
+        const int       q = (int)(item / nb) - b0, j = (int)(item % nb);
+        const double*   d   = reinterpret_cast<const double*>(smraw + mb * q);
+        const double*   e2  = d + n;
+        const float*    df  = reinterpret_cast<const float*>(e2 + n);
+        const float *   e2f = df + n, *dlo = e2f + n, *e2lo = dlo + n;
+        const double    tnorm = share[q].tnorm, pivmin = share[q].pivmin;
+        const float     pivf = share[q].pivf;
+        double          a = share[q].lo, c = share[q].hi;
+        auto below64 = [&](double y) { return sturm_count(d, e2, n, y, pivmin) > j; };
+        // FP32 pre-bracketing: bisect in FP32 (the FP32 pipe is 64x wider on GB300) to ~1e-6
+        // relative, widened by 16 eps32 ||T|| (the backward error of an FP32 Sturm count is a few
+        // eps32 ||T||); then a double-single phase down to a few units of its backward error, widened
+        // by that error. The bracket is kept only if two FP64 counts confirm it, else the FP32 one if
+        // they confirm that, else the whole range.
+        const float tolf = 4.f * FLT_EPSILON * (float)tnorm;
+        float       af = (float)a, cf = (float)c;
+        section<P>(af, cf, it_pre, lane, [&](float y) { return sturm_count(df, e2f, n, y, pivf) > j; },
+                   [&](float y, float z, float m) { return z - y <= tolf || m <= y || m >= z; });
+        const double w   = 16.0 * (double)FLT_EPSILON * tnorm;
+        const double lo2 = max(a, (double)af - w), hi2 = min(c, (double)cf + w);
+        if (lo2 < hi2) {
+            const double ulp_ds = 3.552713678800501e-15 * tnorm;  // 2^-48 ||T||
+            double       ad = lo2, cd = hi2;
+            section<P>(ad, cd, it_pre, lane,
+                       [&](double y) { return sturm_count_ds(df, dlo, e2f, e2lo, n, ds_of(y), pivf) > j; },
+                       [&](double y, double z, double m) { return z - y <= 64.0 * ulp_ds || m <= y || m >= z; });
+            const double lo3 = max(lo2, ad - 16.0 * ulp_ds), hi3 = min(hi2, cd + 16.0 * ulp_ds);
+            if (lo3 < hi3 && confirm<P>(lo3, hi3, lane, below64)) {
+                a = lo3;
+                c = hi3;
+            } else if (confirm<P>(lo2, hi2, lane, below64)) {
                 a = lo2;
                 c = hi2;
-                // double-single phase: bisect down to a few units of its backward error, widen by
-                // that error and keep the bracket only if two FP64 counts confirm it
-                const T ulp_ds = T(3.552713678800501e-15) * tnorm;  // 2^-48 ||T||
-                T       ad = a, cd = c;
-                for (int it = 0; it < it_pre; ++it) {
-                    const T mid = T(0.5) * (ad + cd);
-                    if (cd - ad <= T(64) * ulp_ds || mid <= ad || mid >= cd) break;
-                    if (sturm_count_ds(df, dlo, e2f, e2lo, n, ds_of((double)mid), pivf) > j) cd = mid;
-                    else ad = mid;
-                }
-                const T lo3 = max(a, ad - T(16) * ulp_ds), hi3 = min(c, cd + T(16) * ulp_ds);
-                if (lo3 < hi3 && sturm_count(d, e2, n, lo3, pivmin) <= j && sturm_count(d, e2, n, hi3, pivmin) > j) {
-                    a = lo3;
-                    c = hi3;
-                }
             }
         }
-        // count(a) <= j < count(c) holds throughout; at most ~log2(range / atol) < 200 steps.
-        bool done = false;
-        for (int it = 0; it < it_last && !done; ++it) {
-            const T mid = T(0.5) * (a + c);
-            const T tol = max(atol, T(2) * eps * max(fabs(a), fabs(c)));
-            done        = c - a <= tol || mid <= a || mid >= c;
-            if (done) break;
-            if (sturm_count(d, e2, n, mid, pivmin) > j) c = mid;
-            else a = mid;
+        a0 = a;
+        c0 = c;
+        if constexpr (P != Q) {
+            if ((tid & (P - 1)) == 0) {
+                s_a[x] = a;
+                s_c[x] = c;
+            }
+            __syncthreads();
         }
-        if (!done) {
-            const T mid = T(0.5) * (a + c);
-            done        = c - a <= max(atol, T(2) * eps * max(fabs(a), fabs(c))) || mid <= a || mid >= c;
-        }
-        if (!isfinite(a) || !isfinite(c)) flags |= 2;       // UEPM_K_NONFINITE
-        else if (!done) flags |= 1;                         // UEPM_K_NOCONVERGE
-        evOut[(size_t)b * ev_ld + j] = T(0.5) * (a + c);
     }
-    if (flags && status) atomicOr(status + b, flags);
+    // count(a) <= j < count(c) holds throughout; at most ~log2(range / atol) < 200 steps.
+    if (warp * 32 >= IPB * Q) return;
+    {
+        const int       x    = tid / Q;
+        const long long item = min(item0 + x, last);
+        const int       b = (int)(item / nb), q = b - b0, j = (int)(item % nb);
+        const T*        d      = reinterpret_cast<const T*>(smraw + mb * q);
+        const T*        e2     = d + n;
+        const T         pivmin = (T)share[q].pivmin, atol = eps * (T)share[q].tnorm;
+        T               a, c;
+        if constexpr (sizeof(T) == 4) {
+            a = (T)share[q].lo;
+            c = (T)share[q].hi;
+        } else {
+            a = P == Q ? a0 : s_a[x];
+            c = P == Q ? c0 : s_c[x];
+        }
+        auto            stop = [&](T y, T z, T m) {
+            return z - y <= max(atol, T(2) * eps * max(fabs(y), fabs(z))) || m <= y || m >= z;
+        };
+        bool done = section<Q>(a, c, it_last, lane, [&](T y) { return sturm_count(d, e2, n, y, pivmin) > j; }, stop);
+        if (!done) done = stop(a, c, T(0.5) * (a + c));
+        if ((tid & (Q - 1)) == 0 && item0 + x <= last) {
+            int flags = 0;
+            if (!isfinite(a) || !isfinite(c)) flags = 2;  // UEPM_K_NONFINITE
+            else if (!done) flags = 1;                    // UEPM_K_NOCONVERGE
+            evOut[(size_t)b * ev_ld + j] = T(0.5) * (a + c);
+            if (flags && status) atomicOr(status + b, flags);
+        }
+    }
 }
 
+template <typename T, int P, int Q>
+static bool bisect_launch(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap,
+                          int* status) {
+    constexpr int   IPB   = 32 * kBisectWarpsPerBlock / P;
+    const long long items = (long long)batch * nb;
+    // matrices that IPB consecutive values can touch
+    const int    nm   = std::min(batch, IPB % nb == 0 ? std::max(1, IPB / nb) : (IPB - 1) / nb + 2);
+    const size_t smem = (bisect_matrix_bytes<T>(n) + sizeof(BisectMatrix)) * nm;
+    if (smem > 96 * 1024) return false;
+    auto kern = k_bisect<T, P, Q>;
+    if (smem > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<(unsigned)((items + IPB - 1) / IPB), 32 * kBisectWarpsPerBlock, smem, s>>>(d, e, n, nb, ev, ev_ld, batch, cap,
+                                                                                   status);
+    count_launch();
+    return true;
+}
+
+// Lanes per value. A value is a chain of ~60 Sturm counts of n dependent steps; while the values do not
+// fill the GPU's 608 schedulers a few warps deep, more lanes per value shorten the chain. Measured (values =
+// batch x nb; us with one lane against the choice): FP64 n = 137, 16 values 876 -> 239 (32 lanes), 960
+// 882 -> 266 (16), 3200 883 -> 464 and 8000 883 -> 661 (4), 16000 883 -> 797 (4, then 1 in the FP64 phase),
+// n = 113 24000 1046 -> 760, n = 181 1800 1159 -> 430 (8); FP32 n = 137, 960 98 -> 29 (32), 4800 98 -> 45 (8),
+// 16000 105 -> 86 (4). Beyond the last threshold one lane is fastest (65536 FP64 values: 2091 against 2152).
 template <typename T>
 void launch_bisect(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap, int* status) {
-    // lanes per matrix: >= nb (one lane per eigenvalue) and large enough that the d / e^2 copies
-    // of the warp's matrices fit in 96 KB of shared memory per block
-    const int max_mpw = (int)std::max<size_t>(1, (96 * 1024) / (bisect_matrix_bytes<T>(n) * kBisectWarpsPerBlock));
-    int       lpm     = 1;
-    while ((lpm < nb || 32 / lpm > max_mpw) && lpm < 32) lpm <<= 1;
-    const int    mpw    = 32 / lpm;
-    const int    warps  = (batch + mpw - 1) / mpw;
-    const int    blocks = (warps + kBisectWarpsPerBlock - 1) / kBisectWarpsPerBlock;
-    const size_t smem   = bisect_matrix_bytes<T>(n) * mpw * kBisectWarpsPerBlock;
-    auto         kern   = k_bisect<T>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<blocks, 32 * kBisectWarpsPerBlock, smem, s>>>(d, e, n, nb, lpm, ev, ev_ld, batch, cap, status);
-    count_launch();
+    if (batch <= 0) return;
+    const long long items = (long long)batch * nb;
+#define UEPM_BIS(P_, Q_) bisect_launch<T, P_, Q_>(d, e, n, nb, ev, ev_ld, batch, s, cap, status)
+    if constexpr (sizeof(T) == 8) {
+        if (items > 512 && items <= 1024 && UEPM_BIS(16, 16)) return;
+        if (items > 1024 && items <= 2400 && UEPM_BIS(8, 8)) return;
+        if (items > 2400 && items <= 12000 && UEPM_BIS(4, 4)) return;
+        if (items > 12000 && items <= 40000 && UEPM_BIS(4, 1)) return;
+        if (items > 40000 && UEPM_BIS(1, 1)) return;
+    } else {
+        if (items > 1024 && items <= 6000 && UEPM_BIS(8, 8)) return;
+        if (items > 6000 && items <= 24000 && UEPM_BIS(4, 4)) return;
+        if (items > 24000 && UEPM_BIS(1, 1)) return;
+    }
+    // few values, or orders whose staging leaves room for few matrices per CTA
+    UEPM_BIS(32, 32);
+#undef UEPM_BIS
 }
 
 // ------------------------------------------------------------------------------------------------
