@@ -195,7 +195,7 @@ int uepm_measure_peak(int precision, double* tflops);
 
 /* ---- Tuning (no reference counterpart) -------------------------------------------------------
  * Kernel-shape choices of a context. 0 in a field means "automatic":
- *   reduction     the Householder reduction kernel: 1 register-resident (FP32 real matrices, n <= 176),
+ *   reduction     the Householder reduction kernel: 1 register-resident (FP32 real matrices, n <= 192),
  *                 2 one CTA per matrix (shared memory where the matrix fits, else global memory with
  *                 a persistent grid), 3 one thread-block cluster per matrix, the matrix spread over
  *                 the cluster's shared memory (orders beyond one SM), 4 one CTA per matrix in global

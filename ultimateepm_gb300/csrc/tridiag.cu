@@ -892,6 +892,13 @@ void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d
 template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant, int ctas_per_sm, int cluster, bool tensor_cores) {
+    // complex orders whose lower triangle fits one SM's shared memory and fills it alone: reduction of 1500
+    // matrices in ms, triangular against deferred (5) and blocked (6): n = 178 6.69, 7.45, 8.81; 181 6.76,
+    // 7.78, 8.97; 226 11.06, 13.92, 12.86; 229 11.97, 14.38, 13.11. Below, several deferred CTAs per SM hide
+    // more of the serial chain (2000 matrices, n = 113 3.02 against 2.37, 169 8.74 against 8.15).
+    if constexpr (std::is_same<S, cx<float>>::value)
+        if (variant == 0 && n >= 175 && n <= 230 && launch_tridiag_tri<S>(H, n, ld, mstride, d, e, tq, status, batch, s))
+            return;
     if constexpr (std::is_same<S, float>::value) {
         if ((variant == 0 || variant == 1) && n <= tridiag_reg_max_n()) {
             launch_tridiag_reg(H, n, ld, mstride, d, e, tq, status, batch, s);
@@ -907,11 +914,10 @@ void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, t
     // update deferred, 3 passes per two steps, 5 and automatic). Reduction time per 2000 k: Ge SOC
     // n = 362 222 ms unfused, 102.7 fused, 81.3 deferred; GaP SOC n = 458 230.6 -> 198.3 ms.
     if constexpr (F32) {
-        // the blocked kernel (6) is automatic from order 200 (2000 k, mixed: Ge SOC n = 362 81.3 ->
+        // the blocked kernel (6) is automatic from order 231 (2000 k, mixed: Ge SOC n = 362 81.3 ->
         // 47.5 ms, Si SOC n = 338 67.1 -> 41.7, GaP SOC n = 458 198.3 -> 81.8; with its trailing updates
         // on the tensor cores, whole solves against the deferred kernel: Si SOC n = 274 33.4 against
-        // 45.5 ms, InAs n = 229 27.2 against 27.7); below, the deferred kernel stays ahead (GaAs SOC
-        // n = 178 16.5 against 19.3 ms per solve). Real matrices, whose updates stay on the FP32 pipe,
+        // 45.5 ms, InAs n = 229 27.2 against 27.7). Real matrices, whose updates stay on the FP32 pipe,
         // keep the order-300 switch (real Sn and Ge n = 229: deferred 16.3 and 17.4 ms per solve,
         // blocked 19.4 and 20.6).
         if ((variant == 6 || (variant == 0 && n >= (ST<S>::cplx ? 200 : 300))) &&
