@@ -159,12 +159,20 @@ struct Layout {
 // kernels nor a reduction kernel of the complex matrix is asked for.
 bool quaternionic(const uepm_ctx* ctx) { return ctx->quat_h && !ctx->force_cx && ctx->tune.reduction == 0; }
 
+// Vectors a solve of nb bands carries: with the guard bands in mixed precision, whole Kramers pairs where
+// the matrix is quaternionic.
+int subspace(const uepm_ctx* ctx, int nb) {
+    if (ctx->precision != UEPM_PREC_MIXED) return nb;
+    const int m = std::min(ctx->n, nb + kGuardBands);
+    return quaternionic(ctx) ? (m + 1) & ~1 : m;
+}
+
 // Bytes of workspace one chunk of `c` matrices needs, with the offset of every region.
 Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
     const size_t n = ctx->n, N = ctx->N;
     const bool   mixed = ctx->precision == UEPM_PREC_MIXED;
     const bool   vecs  = (want & (UEPM_WANT_VECTORS | UEPM_WANT_GRADIENT)) != 0;
-    const size_t m     = mixed ? std::min<size_t>(n, (size_t)nb + kGuardBands) : (size_t)nb;
+    const size_t m     = (size_t)subspace(ctx, nb);
     const size_t es    = ctx->real ? sizeof(double) : sizeof(cx<double>);  // FP64 matrix scalar
     const size_t es32  = ctx->real ? sizeof(float) : sizeof(cx<float>);   // FP32 matrix scalar
     const size_t rs    = mixed ? sizeof(float) : sizeof(double);           // real type of the reduction
@@ -387,7 +395,8 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
         ProfScope p(ctx, s, KK_REFINE_PROJECT);
         const SparseV sv{ctx->sparse_local, ctx->ell_w,  ctx->d_ell_col, ctx->d_ell_re,
                          ctx->d_ell_im,       ctx->d_Vloc, rows,            ctx->N};
-        launch_refine_project<S>(Hs, n, n, mstride, X32, m, rw, small, c, s, sv, st, ctx->tune.tensor_cores == 0);
+        launch_refine_project<S>(Hs, n, n, mstride, X32, m, rw, small, c, s, sv, st, ctx->tune.tensor_cores == 0,
+                                 quat ? N : 0);
     }
     S* W = small + (size_t)2 * m * m;  // W block of the first matrix; matrices are refine_small_elems apart
     {
@@ -426,7 +435,7 @@ int plan_solve(uepm_ctx* ctx, size_t nk, int nb, uint32_t want, SolvePlan* out, 
     }
     const bool mixed = ctx->precision == UEPM_PREC_MIXED;
     const int  n     = ctx->n;
-    const int  m     = mixed ? std::min(n, nb + kGuardBands) : nb;
+    const int  m     = subspace(ctx, nb);
     if (mixed && m > kRefineMaxSubspace) {
         set_error("mixed precision supports at most " + std::to_string(kRefineMaxSubspace - kGuardBands) + " bands");
         return UEPM_ERR_INVALID;

@@ -100,7 +100,7 @@ template <typename S, bool STAGED, bool SPARSE, bool YDONE = false>
 __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split<S>::type* __restrict__ H, int n, int ld,
                                                             size_t mstride, const cx<float>* __restrict__ X32, int m,
                                                             void* __restrict__ work, S* __restrict__ small, int batch,
-                                                            const SparseV sv) {
+                                                            const SparseV sv, int nr) {
     constexpr bool CX = !std::is_same<S, double>::value;
     using SE          = typename Split<S>::type;
     using XT          = XElem<S>;
@@ -130,7 +130,10 @@ __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split
     YT*       Y    = reinterpret_cast<YT*>(work) + (size_t)b * refine_work_elems(n, m) * sizeof(S) / sizeof(YT);  // [r][mp]
     const SE* A    = H + (size_t)b * mstride;
     const int nblk = mp / kProjVB;
-    for (int item = tid; item < (YDONE ? 0 : nblk * n); item += kProjNT) {  // YDONE: Y came from the tensor cores
+    // nr < n: a quaternionic H, of which only the first nr = n / 2 rows exist; the vectors are pairs, and the
+    // rows below follow from the pair's other member (Y(r + nr, 2 p) = -conj Y(r, 2 p + 1), Y(r + nr, 2 p + 1) =
+    // conj Y(r, 2 p))
+    for (int item = tid; item < (YDONE ? 0 : nblk * nr); item += kProjNT) {  // YDONE: Y came from the tensor cores
         const int r = item / nblk, jb = item - r * nblk, j0 = jb * kProjVB;
         dsacc     yr[kProjVB], yi[kProjVB];
 #pragma unroll
@@ -153,7 +156,13 @@ __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split
         }
 #pragma unroll
         for (int q = 0; q < kProjVB; ++q) {
-            if constexpr (CX) Y[(size_t)r * mp + j0 + q] = make_float4(yr[q].h, yr[q].l, yi[q].h, yi[q].l);
+            if constexpr (CX) {
+                Y[(size_t)r * mp + j0 + q] = make_float4(yr[q].h, yr[q].l, yi[q].h, yi[q].l);
+                if (nr < n) {
+                    const float sg = q & 1 ? -1.f : 1.f;
+                    Y[(size_t)(r + nr) * mp + j0 + (q ^ 1)] = make_float4(sg * yr[q].h, sg * yr[q].l, -sg * yi[q].h, -sg * yi[q].l);
+                }
+            }
             else Y[(size_t)r * mp + j0 + q] = make_float2(yr[q].h, yr[q].l);
         }
     }
@@ -654,21 +663,23 @@ __global__ void k_refine_vectors(int n, int m, int nb, const cx<float>* __restri
 
 template <typename S, bool SPARSE, bool YDONE>
 static void refine_project_t(const typename Split<S>::type* H, int n, int ld, size_t mstride, const cx<float>* X32, int m,
-                             S* work, S* small, int batch, cudaStream_t s, const SparseV& sv) {
+                             S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int half = 0) {
+    const int    nr    = half ? half : n;
     const size_t stage = proj_stage_bytes<S>(n, m);
     if (stage <= kProjStageBytes) {
         auto kern = k_refine_project<S, true, SPARSE, YDONE>;
         if (stage > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage);
-        kern<<<batch, kProjNT, stage, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv);
+        kern<<<batch, kProjNT, stage, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
     } else {
-        k_refine_project<S, false, SPARSE, YDONE><<<batch, kProjNT, 0, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv);
+        k_refine_project<S, false, SPARSE, YDONE><<<batch, kProjNT, 0, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
     }
     count_launch();
 }
 
 template <typename S>
 void launch_refine_project(const typename Split<S>::type* H, int n, int ld, size_t mstride, const cx<float>* X32, int m,
-                           S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int* status, bool tensor_cores) {
+                           S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int* status, bool tensor_cores,
+                           int half) {
     if (sv.on) {
         refine_project_t<S, true, false>(H, n, ld, mstride, X32, m, work, small, batch, s, sv);
         return;
@@ -679,12 +690,13 @@ void launch_refine_project(const typename Split<S>::type* H, int n, int ld, size
         // complex multiply-adds per element there, the tensor-core form's slicing and second pass over
         // H do not pay (Ge nonlocal n = 181, 2000 k: 0.96 ms against 0.83)
         if (tensor_cores && n >= kRefineTcMinN &&
-            launch_refine_y_tc(H, n, ld, mstride, X32, m, proj_mp<S>(m), work, refine_work_elems(n, m), status, batch, s)) {
+            launch_refine_y_tc(H, n, ld, mstride, X32, m, proj_mp<S>(m), work, refine_work_elems(n, m), status, batch, s,
+                               half)) {
             refine_project_t<S, false, true>(H, n, ld, mstride, X32, m, work, small, batch, s, sv);
             return;
         }
     }
-    refine_project_t<S, false, false>(H, n, ld, mstride, X32, m, work, small, batch, s, sv);
+    refine_project_t<S, false, false>(H, n, ld, mstride, X32, m, work, small, batch, s, sv, half);
 }
 
 template <typename S>
@@ -706,7 +718,7 @@ void launch_refine_vectors(int n, int m, int nb, const cx<float>* X32, const S* 
 
 #define UEPM_RF_INST(S)                                                                                             \
     template void launch_refine_project<S>(const typename Split<S>::type*, int, int, size_t, const cx<float>*, int, S*, S*, \
-                                           int, cudaStream_t, const SparseV&, int*, bool);                        \
+                                           int, cudaStream_t, const SparseV&, int*, bool, int);                        \
     template void launch_small_eigh<S>(S*, int, int, double*, S*, int*, int, cudaStream_t, int);                   \
     template void launch_refine_vectors<S>(int, int, int, const cx<float>*, const S*, cx<double>*, double*, const DevParams&, \
                                            const double*, const int*, int, cudaStream_t);

@@ -23,6 +23,10 @@
 // Im Y(r, j). K is walked in chunks of 16 complex columns (K 32: their Re parts, then their Im
 // parts).
 //
+// Quaternionic H (half = N rows computed): with the vectors in pairs (a, -conj b), (b, conj a), the first
+// N rows of Y hold all of it, Y(r + N, 2 p) = -conj Y(r, 2 p + 1) and Y(r + N, 2 p + 1) = conj Y(r, 2 p), and
+// only the first N rows of H exist. Ge (N = 181): 2 row tiles instead of 3 per matrix.
+//
 // One CTA (512 threads) per 128-row tile of one matrix: a pass over the tile's rows for their
 // scales (and over X for the vectors'), then the chunks pipelined over two operand buffers: warps
 // 1..15 slice chunk q into buffer q & 1 (after the MMAs of chunk q - 2 released it) and signal an
@@ -104,7 +108,7 @@ __device__ __forceinline__ void scale_of(float x, float& mul, int& E) {
 
 __global__ void __launch_bounds__(kYtNT, 1)
     k_refine_y_tc(const ds4* __restrict__ H, int n, int ld, size_t mstride, const cx<float>* __restrict__ X32, int m,
-                  int mp, int N, float4* __restrict__ Yw, size_t ystride, int* __restrict__ status, int ntile) {
+                  int mp, int N, float4* __restrict__ Yw, size_t ystride, int* __restrict__ status, int ntile, int nr) {
     extern __shared__ __align__(1024) unsigned char smraw[];
     __shared__ float    s_rmax[kYtM], s_rmul[kYtM], s_cmax[kYtNmax / 2], s_cmul[kYtNmax / 2];
     __shared__ int      s_rE[kYtM], s_cE[kYtNmax / 2];
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(kYtNT, 1)
         const int     rl = tid & (kYtM - 1), part = tid >> 7, r = r0 + rl;
         const float4* Af = reinterpret_cast<const float4*>(A);  // (rhi, rlo, ihi, ilo)
         float         mx = 0.f;
-        if (r < n) {
+        if (r < nr) {
             int c = part;
             for (; c + (kYtPass - 1) * kStep < n; c += kYtPass * kStep) {
                 float4 v[kYtPass];
@@ -193,7 +197,7 @@ __global__ void __launch_bounds__(kYtNT, 1)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int c = c0 + 8 * h + i;
-                        const ds4 v = (r < n && c < n) ? A[(size_t)c * ld + r] : ds4{0.f, 0.f, 0.f, 0.f};
+                        const ds4 v = (r < nr && c < n) ? A[(size_t)c * ld + r] : ds4{0.f, 0.f, 0.f, 0.f};
                         pr[i]       = v.rhi * mu;  // powers of two: exact
                         qr[i]       = v.rlo * mu;
                         pi[i]       = v.ihi * mu;
@@ -288,7 +292,7 @@ __global__ void __launch_bounds__(kYtNT, 1)
                         l[i] = __fadd_rn(l[i], x);
                     }
                 }
-                if (r < n) {
+                if (r < nr) {
                     float* Yr = reinterpret_cast<float*>(Yw + (size_t)b * ystride + (size_t)r * mp);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
@@ -299,8 +303,16 @@ __global__ void __launch_bounds__(kYtNT, 1)
                         const int  e   = s_rE[r - r0] + s_cE[j] - 12;
                         float      hh = h[i], ll = l[i];
                         two_sum(hh, ll);  // renormalised pair
-                        Yr[(size_t)j * 4 + (imr ? 2 : 0)] = ldexpf(hh, e);
-                        Yr[(size_t)j * 4 + (imr ? 3 : 1)] = ldexpf(ll, e);
+                        hh = ldexpf(hh, e);
+                        ll = ldexpf(ll, e);
+                        Yr[(size_t)j * 4 + (imr ? 2 : 0)] = hh;
+                        Yr[(size_t)j * 4 + (imr ? 3 : 1)] = ll;
+                        if (nr < n) {  // row r + nr of the pair's other member: conj, negated under an odd j
+                            const float sg = (imr != ((j & 1) != 0)) ? -1.f : 1.f;
+                            float*      Yb = Yr + ((size_t)nr * mp + (j ^ 1)) * 4;
+                            Yb[imr ? 2 : 0] = sg * hh;
+                            Yb[imr ? 3 : 1] = sg * ll;
+                        }
                     }
                 }
             }
@@ -319,14 +331,15 @@ __global__ void __launch_bounds__(kYtNT, 1)
 }  // namespace
 
 bool launch_refine_y_tc(const ds4* H, int n, int ld, size_t mstride, const cx<float>* X32, int m, int mp, void* work,
-                        size_t ystride, int* status, int batch, cudaStream_t s) {
+                        size_t ystride, int* status, int batch, cudaStream_t s, int half) {
     const int N = (2 * mp + 15) / 16 * 16;
     if (n < 2 || n > 1024 || m > mp || N > kYtNmax || mp > kYtNmax / 2) return false;
     auto kern = k_refine_y_tc;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYtSmem) != cudaSuccess) return false;
-    const int ntile = (n + kYtM - 1) / kYtM;
+    const int nr    = half ? half : n;
+    const int ntile = (nr + kYtM - 1) / kYtM;
     kern<<<batch * ntile, kYtNT, kYtSmem, s>>>(H, n, ld, mstride, X32, m, mp, N, reinterpret_cast<float4*>(work), ystride,
-                                              status, ntile);
+                                              status, ntile, nr);
     count_launch();
     return true;
 }

@@ -141,17 +141,19 @@ struct SparseV {
     const double*     rows;  // [batch][N][ROW_STRIDE], for the kinetic term
     int               N;
 };
+// half > 0: H is quaternionic, only its first half = n / 2 rows are formed, and the vectors come in pairs
+// (launch_backtransform_quat's); the other rows of Y follow from those.
 // tensor_cores: a complex dense H of order >= kRefineTcMinN takes Y = H X on the tensor cores
 // (refine_tc.cu); status gets UEPM_K_NOCONVERGE there if a bounded wait gives up.
 constexpr int kRefineTcMinN = 150;
 template <typename S>
 void launch_refine_project(const typename Split<S>::type* H, int n, int ld, size_t mstride, const cx<float>* X32, int m,
                            S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int* status = nullptr,
-                           bool tensor_cores = true);
+                           bool tensor_cores = true, int half = 0);
 // refine_tc.cu: Y (double-single, [r][mp] per matrix, ystride float4 apart) = H X for complex H on
 // the tensor cores; false when it does not apply (nothing launched).
 bool launch_refine_y_tc(const ds4* H, int n, int ld, size_t mstride, const cx<float>* X32, int m, int mp, void* work,
-                        size_t ystride, int* status, int batch, cudaStream_t s);
+                        size_t ystride, int* status, int batch, cudaStream_t s, int half = 0);
 template <typename S>
 void launch_small_eigh(S* small, int m, int nb, double* Eout, S* W, int* status, int batch, cudaStream_t s, int cap = 0);
 template <typename S>
