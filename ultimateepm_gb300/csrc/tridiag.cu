@@ -25,354 +25,11 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "tridiag_kernel.cuh"
 #include "uepm_common.cuh"
 #include "uepm_kernels.h"
 
 namespace uepm {
-
-constexpr int kUpd = 4;  // elements per thread per round of the rank-2 update
-
-// SMEM = true: the matrix is copied into shared memory (leading dimension n | 1, odd, so that the
-// mirrored row-wise stores do not collide on banks), reduced there, and its reflector columns are
-// written back. Used where n x n fits (the FP32 reductions of the mixed path), because those are
-// bound by memory latency rather than by arithmetic.
-// Global-memory variant: CTAs per SM that must fit the register file (the persistent grid relies on
-// several to hide L2/DRAM latency): 5 for the real and complex-FP32 matrices up to n = 161, 4 above,
-// fewer for complex FP64 with many row chunks (whose accumulators alone take 4 MAXT registers).
-template <typename S, int MAXT>
-constexpr int tridiag_min_blocks() {
-    return is_quat<S>::value ? 2 : sizeof(S) * MAXT <= 8 * 5 ? 5 : (sizeof(S) <= 8 || MAXT <= 5 ? 4 : (MAXT <= 8 ? 3 : 2));
-}
-
-template <typename T>
-__device__ __forceinline__ T shfl_xor(T a, int o) {
-    return __shfl_xor_sync(0xffffffffu, a, o);
-}
-template <typename T>
-__device__ __forceinline__ cx<T> shfl_xor(cx<T> a, int o) {
-    return mk(shfl_xor(a.x, o), shfl_xor(a.y, o));
-}
-template <typename T>
-__device__ __forceinline__ qt<T> shfl_xor(qt<T> a, int o) {
-    return mkq(shfl_xor(a.w, o), shfl_xor(a.x, o), shfl_xor(a.y, o), shfl_xor(a.z, o));
-}
-
-// zlarfg's scalars of the column (c0; tail), tail2 = |tail|^2: beta real, th = (beta - c0) / beta,
-// sc = 1 / (c0 - beta). One division serves both reciprocals (an FP64 division costs as much of the
-// FP64 pipe as a 30-row column of the product) while the products stay well inside the exponent range.
-template <typename S>
-__device__ __forceinline__ void reflector_scalars(S c0, typename ST<S>::R tail2, typename ST<S>::R& beta, S& th, S& sc) {
-    using R = typename ST<S>::R;
-    if constexpr (is_quat<S>::value) {
-        quat_reflector(c0, tail2, num<R>::tiny(), beta, th, sc);
-    } else {
-        const R c0r = ST<S>::re(c0), c0i = ST<S>::im(c0);
-        if (tail2 <= num<R>::tiny() && c0i * c0i <= num<R>::tiny()) {
-            th   = ST<S>::zero();
-            sc   = ST<S>::zero();
-            beta = c0r;
-            return;
-        }
-        beta = sqrt(fma(c0r, c0r, fma(c0i, c0i, tail2)));
-        if (c0r >= 0) beta = -beta;
-        const R ar = c0r - beta, q = fma(ar, ar, c0i * c0i);
-        R       ib, den;
-        const float mag = fabsf((float)beta);
-        if (sizeof(R) == 8 && mag > 1e-30f && mag < 1e30f) {
-            const R inv = R(1) / (beta * q);
-            ib          = inv * q;
-            den         = inv * beta;
-        } else {
-            ib  = R(1) / beta;
-            den = R(1) / q;
-        }
-        th = ST<S>::make((beta - c0r) * ib, -c0i * ib);
-        sc = ST<S>::make(ar * den, -c0i * den);
-    }
-}
-
-// pw[r] = this warp's part of (A v)_r over its columns (c = warp mod NW), A full, m x m: lanes own rows.
-// TF full 32-row chunks; the remaining rows take one instruction for 1, 2 or 4 columns (a lane group of
-// 32, 16 or 8 lanes each). The chunk count is a template parameter, so that no dead chunk is issued:
-// predicated off they still took the FP64 pipe (91 k instructions per matrix at n = 137, 70 k so).
-template <typename S, int NW, int TF>
-__device__ __forceinline__ void product_t(const S* __restrict__ A, int ld, int m, const S* v, S* pw, int warp, int lane) {
-    if constexpr (TF > 0) {
-        S acc[TF];
-#pragma unroll
-        for (int t = 0; t < TF; ++t) acc[t] = ST<S>::zero();
-        const int tf = m >> 5;
-        for (int c = warp; c < m; c += NW) {
-            const S* ac = A + (size_t)c * ld + lane;
-            const S  vc = v[c];
-            S        a[TF];
-#pragma unroll
-            for (int t = 0; t < TF; ++t) a[t] = TF <= 8 || t < tf ? ldc(ac + 32 * t) : ST<S>::zero();
-#pragma unroll
-            for (int t = 0; t < TF; ++t) acc[t] = cfma(a[t], vc, acc[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < TF; ++t)
-            if (TF <= 8 || t < tf) pw[lane + 32 * t] = acc[t];
-    }
-    const int rem = m & 31;
-    if (rem) {
-        const int lg = rem <= 8 ? 3 : rem <= 16 ? 4 : 5, g = 32 >> lg;  // 2^lg lanes per column
-        const int sub = lane >> lg, rr = (m & ~31) + (lane & ((1 << lg) - 1));
-        const S*  ar = A + rr;
-        S         at = ST<S>::zero();
-        int       c0 = warp * g;
-        for (; c0 + 3 * NW * g + g <= m; c0 += 4 * NW * g) {
-            S a[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) a[q] = rr < m ? ldc(ar + (size_t)(c0 + q * NW * g + sub) * ld) : ST<S>::zero();
-#pragma unroll
-            for (int q = 0; q < 4; ++q) at = cfma(a[q], v[c0 + q * NW * g + sub], at);
-        }
-        for (; c0 < m; c0 += NW * g) {
-            const int c = c0 + sub;
-            if (c0 + g <= m || c < m) at = cfma(rr < m ? ldc(ar + (size_t)c * ld) : ST<S>::zero(), v[c], at);
-        }
-        for (int q = 16; q >= (1 << lg); q >>= 1) at = cadd(at, shfl_xor(at, q));
-        if (sub == 0 && rr < m) pw[rr] = at;
-    }
-}
-template <typename S, int NW, int MAXT>
-__device__ __forceinline__ void product(const S* A, int ld, int m, const S* v, S* pw, int warp, int lane) {
-    switch (m >> 5) {
-        case 0: product_t<S, NW, 0>(A, ld, m, v, pw, warp, lane); break;
-        case 1: product_t<S, NW, 1>(A, ld, m, v, pw, warp, lane); break;
-        case 2: product_t<S, NW, 2>(A, ld, m, v, pw, warp, lane); break;
-        case 3: product_t<S, NW, 3>(A, ld, m, v, pw, warp, lane); break;
-        case 4: if constexpr (MAXT >= 4) product_t<S, NW, 4>(A, ld, m, v, pw, warp, lane); break;
-        case 5: if constexpr (MAXT >= 5) product_t<S, NW, 5>(A, ld, m, v, pw, warp, lane); break;
-        case 6: if constexpr (MAXT >= 6) product_t<S, NW, 6>(A, ld, m, v, pw, warp, lane); break;
-        case 7: if constexpr (MAXT >= 7) product_t<S, NW, 7>(A, ld, m, v, pw, warp, lane); break;
-        case 8: if constexpr (MAXT >= 8) product_t<S, NW, 8>(A, ld, m, v, pw, warp, lane); break;
-        case 9: case 10: case 11:
-        case 12: if constexpr (MAXT >= 12) product_t<S, NW, 12>(A, ld, m, v, pw, warp, lane); break;
-        default: if constexpr (MAXT >= 16) product_t<S, NW, 16>(A, ld, m, v, pw, warp, lane); break;
-    }
-}
-
-template <typename S, int NT, int MAXT, bool SMEM>
-__global__ void __launch_bounds__(NT, SMEM ? 1 : tridiag_min_blocks<S, MAXT>()) k_tridiag(S* __restrict__ H, int n, int ldg, size_t mstride,
-                                                typename ST<S>::R* __restrict__ dOut, typename ST<S>::R* __restrict__ eOut,
-                                                S* __restrict__ tqOut, int* __restrict__ status, int batch) {
-    using R       = typename ST<S>::R;
-    constexpr int NW = NT / 32;
-    const int lds = n | 1;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    S*        As   = reinterpret_cast<S*>(smraw);  // SMEM: n x lds
-    S*        v    = SMEM ? As + (size_t)n * lds : As;  // n
-    S*        w    = v + n;                        // n
-    S*        pacc = w + n;                        // NW * n
-    __shared__ S   s_th, s_sc, red2[NW];
-    __shared__ R   red[NW];
-    __shared__ int s_skip;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // The grid may be smaller than the batch: each CTA reduces matrices b, b + gridDim.x, ... so the
-    // number of matrices in flight (and their L2 working set) is set by the launch, not the batch.
-    for (int b = blockIdx.x; b < batch; b += gridDim.x) {
-    S*        Ag  = H + (size_t)b * mstride;
-    bool      bad = false;
-    S*        A   = SMEM ? As : Ag;
-    const int ld  = SMEM ? lds : ldg;
-    if (SMEM) {
-        for (int q = tid; q < n * n; q += NT) {
-            const int c = q / n, r = q - c * n;
-            As[(size_t)c * lds + r] = Ag[(size_t)c * ldg + r];
-        }
-        __syncthreads();
-    }
-
-    // xc: this thread's rows (tid, tid + NT) of the column to reduce next, and ss their norm's sum over
-    // the tail; from the matrix for column 0, from the previous column's update afterwards
-    S xc[2];
-    R ss = 0;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int r = tid + k * NT;  // row o + r - 1 of column 0: r = 0 is the diagonal
-        xc[k]       = r < n ? ldc(A + r) : ST<S>::zero();
-        if (r >= 2 && r < n) ss += ST<S>::norm(xc[k]);
-    }
-    for (int i = 0; i < n - 1; ++i) {
-        const int o = i + 1, m = n - o;
-        S*        col = A + (size_t)i * ld + o;
-
-        // ---- Householder vector of A[o:, i] -------------------------------------------------
-        // The column's rows are in the registers of the threads that updated it (thread r: row i + r),
-        // so nothing is read back, and each warp that holds some sums its squares.
-        if (32 * warp <= m) {
-            ss = warp_sum(ss);
-            if (lane == 0) red[warp] = ss;
-        }
-        if (tid == 1) s_sc = xc[0];  // c0
-        __syncthreads();
-        if (warp == 0) {
-            R tail2 = red[0];
-            for (int q = 1; q < NW && 32 * q <= m; ++q) tail2 += red[q];
-            R beta;
-            S th, sc;
-            reflector_scalars(s_sc, tail2, beta, th, sc);
-            __syncwarp();
-            if (lane == 0) {
-                const R di = ST<S>::re(xc[0]);
-                s_th   = th;
-                s_sc   = sc;
-                s_skip = ST<S>::norm(th) == R(0);
-                dOut[(size_t)b * n + i]  = di;
-                eOut[(size_t)b * n + i]  = beta;
-                tqOut[(size_t)b * n + i] = th;
-                stc(col, ST<S>::make(beta, R(0)));
-                if (!isfinite(beta) || !isfinite(di)) bad = true;
-            }
-        }
-        __syncthreads();
-        const S th = s_th, sc = s_sc;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int r = tid + k * NT - 1;
-            if (r >= 0 && r < m) {
-                const S vr = r == 0 ? ST<S>::one() : cmul(xc[k], sc);
-                v[r]       = vr;
-                if (r > 0) stc(col + r, vr);
-            }
-        }
-        __syncthreads();
-        ss = 0;
-        if (s_skip) {  // the next column as it stands
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int r = tid + k * NT;
-                xc[k]       = r < m ? ldc(A + (size_t)o * ld + o + r) : ST<S>::zero();
-                if (r >= 2 && r < m) ss += ST<S>::norm(xc[k]);
-            }
-            __syncthreads();
-            continue;
-        }
-
-        // ---- p = A22 v (full storage): warps own columns, lanes own rows ----------------------
-        product<S, NW, MAXT>(A + (size_t)o * ld + o, ld, m, v, pacc + warp * n, warp, lane);
-        __syncthreads();
-
-        // ---- w = tau p; alpha = -tau/2 (w^H v) -------------------------------------------------
-        S wr[2], part2 = ST<S>::zero();
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int r = tid + k * NT;
-            wr[k]       = ST<S>::zero();
-            if (r < m) {
-                S p = pacc[r];
-#pragma unroll
-                for (int q = 1; q < NW; ++q) p = cadd(p, pacc[q * n + r]);
-                if constexpr (is_quat<S>::value) {  // w = p tau, and Re(v^H p)
-                    wr[k] = cmul(p, th);
-                    part2.w += re_dot(v[r], p);
-                } else {
-                    wr[k] = cmul(th, p);
-                    part2 = cfmac(wr[k], v[r], part2);
-                }
-            }
-        }
-        if (32 * warp < m) {
-            if constexpr (ST<S>::cplx) {
-                part2 = warp_sum(part2);
-            } else {
-                part2 = ST<S>::make(warp_sum(ST<S>::re(part2)), R(0));
-            }
-            if (lane == 0) red2[warp] = part2;
-        }
-        __syncthreads();
-        if (32 * warp < m) {
-            S wv = red2[0];
-            for (int q = 1; q < NW && 32 * q < m; ++q) {
-                if constexpr (is_quat<S>::value) wv.w += red2[q].w;
-                else wv = cadd(wv, red2[q]);
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int r = tid + k * NT;
-                if (r < m) {
-                    if constexpr (is_quat<S>::value)  // v^H A v is real: -|tau|^2 (v^H p) / 2
-                        w[r] = cadd(wr[k], cscale(v[r], R(-0.5) * wv.w * ST<S>::norm(th)));
-                    else w[r] = cfma(cscale(cmul(th, wv), R(-0.5)), v[r], wr[k]);
-                }
-            }
-        }
-        __syncthreads();
-
-        // ---- A22 -= v w^H + w v^H: lower triangle computed, upper mirrored -------------------
-        // The m (m + 1) / 2 lower elements in column-major order, element e to thread e mod NT:
-        // consecutive threads take consecutive rows of a column (coalesced), and only the last
-        // round has idle lanes (per-column 32-row chunks left ~16 idle lanes in every column).
-        // Each thread takes its elements kUpd at a time, all loads first, so that kUpd loads per
-        // thread are in flight (one at a time left every element waiting a full L2/DRAM latency).
-        // The first m elements are the next column to reduce: they stay in xc.
-        {
-            const int tot = m * (m + 1) / 2;
-            int       c = 0, r = tid;  // (column, row) of element tid
-            while (r >= m && c < m) {
-                r = r - m + c + 1;
-                ++c;
-            }
-            xc[0] = xc[1] = ST<S>::zero();
-            for (int e0 = tid; e0 < tot; e0 += kUpd * NT) {
-                int cq[kUpd], rq[kUpd];
-                S   aq[kUpd];
-#pragma unroll
-                for (int q = 0; q < kUpd; ++q) {
-                    cq[q] = c;
-                    rq[q] = r;
-                    r += NT;  // next element of this thread
-                    while (r >= m && c < m) {
-                        r = r - m + c + 1;
-                        ++c;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kUpd; ++q)
-                    if (e0 + q * NT < tot) aq[q] = ldc(A + (size_t)(o + cq[q]) * ld + o + rq[q]);
-#pragma unroll
-                for (int q = 0; q < kUpd; ++q) {
-                    if (e0 + q * NT >= tot) break;
-                    const int cc = cq[q], rr = rq[q];
-                    S         a  = cfms_conjb(v[rr], w[cc], aq[q]);
-                    a            = cfms_conjb(w[rr], v[cc], a);
-                    if (rr == cc) {
-                        a = ST<S>::make(ST<S>::re(a), R(0));
-                    } else {
-                        stc(A + (size_t)(o + rr) * ld + (o + cc), ST<S>::conj(a));
-                    }
-                    stc(A + (size_t)(o + cc) * ld + o + rr, a);
-                    if (q < 2 && cc == 0) {  // e0 = tid: rows tid and tid + NT of the next column
-                        xc[q] = a;
-                        if (rr >= 2) ss += ST<S>::norm(a);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        const R dl = ST<S>::re(xc[0]);
-        dOut[(size_t)b * n + n - 1] = dl;
-        eOut[(size_t)b * n + n - 1] = R(0);
-        tqOut[(size_t)b * n + n - 1] = ST<S>::zero();
-        if (!isfinite(dl)) bad = true;
-        if (bad && status) atomicOr(status + b, 2);  // UEPM_K_NONFINITE
-    }
-    if (SMEM) {
-        // reflector tails (column i, rows i+2..n-1) for the back-transformation
-        __syncthreads();
-        for (int q = tid; q < n * n; q += NT) {
-            const int c = q / n, r = q - c * n;
-            if (r > c + 1) Ag[(size_t)c * ldg + r] = As[(size_t)c * lds + r];
-        }
-    }
-    __syncthreads();  // shared memory is reused by the CTA's next matrix
-    }
-}
 
 // ------------------------------------------------------------------------------------------------
 // Fused variant for FP32 matrices reduced from L2/DRAM (beyond the on-chip sizes), where every
@@ -884,6 +541,7 @@ static void tridiag_pick(S* H, int n, int ld, size_t mstride, typename ST<S>::R*
 void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d, double* e, qt<double>* tq, int* status,
                          int batch, cudaStream_t s, int ctas_per_sm) {
     using S = qt<double>;
+    if (ctas_per_sm == 0 && launch_tridiag_wide<S>(H, n, ld, mstride, d, e, tq, status, batch, s)) return;
     if (n <= 128) tridiag_launch_t<S, 256, 4, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
     else if (n <= 192) tridiag_launch_t<S, 256, 6, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
     else tridiag_launch_t<S, 256, 8, false>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
@@ -946,6 +604,8 @@ void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, t
         }
     }
     // rows of the trailing matrix are at most n - 1 <= 32 * MAXT
+    if constexpr (!F32)
+        if (variant == 0 && ctas_per_sm == 0 && launch_tridiag_wide<S>(H, n, ld, mstride, d, e, tq, status, batch, s)) return;
     if (n <= 129) tridiag_pick<S, 4>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
     else if (n <= 161) tridiag_pick<S, 5>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
     else if (n <= 257) tridiag_pick<S, 8>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);

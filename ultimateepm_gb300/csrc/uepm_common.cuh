@@ -238,6 +238,46 @@ template <typename T>
 __device__ __forceinline__ T re_dot(qt<T> a, qt<T> b) {
     return fma(a.w, b.w, fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)));
 }
+// sqrt(x) and its reciprocal, and 1 / x. FP64: PTX's approximations (relative error at most 2^-19.9 over 4 M
+// values of all exponents) refined by one step of third order, with e = 1 - x y^2 and y (1 + e/2 + 3 e^2/8) (the binomial
+// series of (1 - e)^-1/2), and e = 1 - x r and r (1 + e + e^2); the square root gets one correction by its
+// residual. Errors of the third order are below 2^-58; what remains is the rounding of the last operations
+// (relative errors at most 1.11e-16, 1.38e-16 and 1.11e-16 over those values). A dependent FP64 operation takes
+// above 100 clocks on this pipe: the reflector's scalars took 4.9 k clocks per column with the library's square
+// root and division and FP64 compares, 3.5 k so. Only where x and its approximation are normal numbers well
+// inside the range (in_seed_range); elsewhere the library's.
+__device__ __forceinline__ bool in_seed_range(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;  // biased exponent
+    return e > 200 && e < 1800;
+}
+__device__ __forceinline__ void sqrt_pair(double x, double& s, double& is) {  // x > 0
+    if (!in_seed_range(x)) {
+        s  = sqrt(x);
+        is = 1.0 / s;
+        return;
+    }
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = x * y;
+    const double e = fma(-t, y, 1.0);
+    const double c = e * fma(0.375, e, 0.5);
+    const double b = fma(t, c, t);
+    is             = fma(y, c, y);
+    s              = fma(0.5 * is, fma(-b, b, x), b);
+}
+__device__ __forceinline__ double recip(double x) {
+    if (!in_seed_range(x)) return 1.0 / x;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ void sqrt_pair(float x, float& s, float& is) {
+    s  = sqrtf(x);
+    is = 1.f / s;
+}
+__device__ __forceinline__ float recip(float x) { return 1.f / x; }
+
 // The reflector of a quaternion column (alpha; tail), |tail|^2 = tail2: H = I - v tau v^H with beta real,
 // tau = (beta - alpha) / beta and v = (1; tail sc), sc = (alpha - beta)^-1 (zlarfg's, the operands in order).
 template <typename T>
@@ -246,11 +286,15 @@ __device__ __forceinline__ void quat_reflector(qt<T> alpha, T tail2, T tiny, T& 
     beta = alpha.w;
     tau = sc = mkq<T>(0, 0, 0, 0);
     if (tail2 <= tiny && im <= tiny) return;
-    beta = sqrt(fma(alpha.w, alpha.w, tail2 + im));
-    if (alpha.w >= 0) beta = -beta;
+    T ib;
+    sqrt_pair(fma(alpha.w, alpha.w, tail2 + im), beta, ib);
+    if (alpha.w >= 0) {
+        beta = -beta;
+        ib   = -ib;
+    }
     const qt<T> df = mkq(alpha.w - beta, alpha.x, alpha.y, alpha.z);
-    tau            = cscale(df, T(-1) / beta);
-    sc             = cscale(mkq(df.w, -df.x, -df.y, -df.z), T(1) / ST<qt<T>>::norm(df));
+    tau            = cscale(df, -ib);
+    sc             = cscale(mkq(df.w, -df.x, -df.y, -df.z), recip(ST<qt<T>>::norm(df)));
 }
 
 // Lower-precision counterpart of a scalar type (FP64 -> FP32), for the mixed path.

@@ -55,6 +55,11 @@ template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant = 0, int ctas_per_sm = 0, int cluster = 0,
                     bool tensor_cores = true);
+// tridiag_wide.cu: the FP64 reduction with a cluster of CTAs per matrix, for few matrices (false, with nothing
+// launched, where that does not pay).
+template <typename S>
+bool launch_tridiag_wide(S* H, int n, int ld, size_t mstride, double* d, double* e, S* tq, int* status, int batch,
+                         cudaStream_t s);
 // The FP64 reduction of quaternion matrices (order n <= 256; tridiag.cu).
 void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d, double* e, qt<double>* tq, int* status,
                          int batch, cudaStream_t s, int ctas_per_sm);
