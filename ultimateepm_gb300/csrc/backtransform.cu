@@ -294,4 +294,25 @@ void launch_pair_values(const double* ev, int nz, double* E, int nb, int batch, 
     count_launch();
 }
 
+__global__ void k_spin_pairs(const double* __restrict__ E, const cx<double>* __restrict__ X, const double* __restrict__ g,
+                             int N, int nf, int nb, double* __restrict__ Eo, cx<double>* __restrict__ Xo,
+                             double* __restrict__ go) {
+    const size_t b = blockIdx.x;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+        Eo[b * nb + i] = E[b * nf + i / 2];
+        if (g)
+            for (int q = 0; q < 3; ++q) go[(b * nb + i) * 3 + q] = g[(b * nf + i / 2) * 3 + q];
+    }
+    if (!X) return;
+    for (int e = threadIdx.x; e < nb * 2 * N; e += blockDim.x) {
+        const int i = e / (2 * N), r = e - i * 2 * N, spin = r >= N;
+        stc(Xo + b * nb * 2 * N + e, spin == (i & 1) ? ldc(X + (b * nf + i / 2) * N + (r - spin * N)) : mk(0.0, 0.0));
+    }
+}
+void launch_spin_pairs(const double* E, const cx<double>* X, const double* g, int N, int nf, int nb, int batch, double* Eo,
+                       cx<double>* Xo, double* go, cudaStream_t s) {
+    k_spin_pairs<<<batch, X ? 256 : 64, 0, s>>>(E, X, g, N, nf, nb, Eo, Xo, go);
+    count_launch();
+}
+
 }  // namespace uepm

@@ -41,13 +41,13 @@ namespace {
         }                                                                              \
     } while (0)
 
-using TuneKey = std::tuple<int, int, int, int, int, int>;  // device, n, real, precision, nb, vectors
+using TuneKey = std::tuple<int, int, int, int, int, int, int>;  // device, n, real, form, precision, nb, vectors
 std::mutex                         g_tune_mu;
 std::map<TuneKey, uepm_tuning>     g_tune_cache;
 
 TuneKey tune_key(const uepm_ctx* ctx, int nb, uint32_t want) {
     const int vec = (want & (UEPM_WANT_VECTORS | UEPM_WANT_GRADIENT)) != 0;
-    return TuneKey{ctx->device, ctx->n, ctx->real ? 1 : 0, ctx->precision, nb, vec};
+    return TuneKey{ctx->device, ctx->n, ctx->real ? 1 : 0, solve_form(ctx), ctx->precision, nb, vec};
 }
 
 bool valid_tuning(const uepm_ctx* ctx, const uepm_tuning& t) {
@@ -426,8 +426,7 @@ int uepm_batch_run(uepm_batch* b, void* stream) {
     for (size_t g = 0; g < order.size(); ++g) order[g] = g;
     auto cost = [&](size_t g) {
         const auto&  gr = b->groups[g];
-        const double n  = (double)gr.ctx->n;
-        return n * n * n * (double)gr.nk * (gr.ctx->real ? 1.0 : 4.0);
+        return reduction_cost(gr.ctx) * (double)gr.nk;
     };
     std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return cost(x) > cost(y); });
     for (size_t q = 0; !rc && q < order.size(); ++q) {

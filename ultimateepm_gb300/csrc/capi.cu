@@ -152,29 +152,51 @@ void pp_value(const uepm_material& m, int gx, int gy, int gz, double tau, double
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct Layout {
-    size_t rows, rows32, H, H32, d, e, tq, ev, work, z, X32, refine, small, total;
+    size_t rows, rows32, H, H32, d, e, tq, ev, work, z, X32, refine, small, fE, fX, fg, total;
 };
 
-// Whether a solve reduces the quaternion form of H(k): where the matrix has it and neither the complex
-// kernels nor a reduction kernel of the complex matrix is asked for.
-bool quaternionic(const uepm_ctx* ctx) { return ctx->quat_h && !ctx->force_cx && ctx->tune.reduction == 0; }
+// The form of H(k) that a solve works on. An explicit reduction kernel, or the complex kernels, work on the
+// full matrix as it stands.
+//   scalar:     a spin-orbit context without spin-orbit strength, H = diag(h, h): the scalar matrix h (order N),
+//               each level and vector for both spins
+//   quaternion: spin-orbit without an antisymmetric part (capi.cu's uepm_ctx_create), order N
+struct Form {
+    bool scalar, quat, real;
+    int  n;       // order of the matrix that is assembled and projected
+    bool ds_nl, ds_soc, sparse;
+};
+Form form_of(const uepm_ctx* ctx) {
+    const bool own = !ctx->force_cx && ctx->tune.reduction == 0;
+    Form       f{};
+    f.scalar = own && ctx->decoupled;
+    f.quat   = own && !f.scalar && ctx->quat_h;
+    f.real   = f.scalar ? ctx->scalar_real : ctx->real;
+    f.n      = f.scalar ? ctx->N : ctx->n;
+    f.ds_nl  = f.scalar ? ctx->scalar_ds_nl : ctx->ds_nl;
+    f.ds_soc = !f.scalar && ctx->ds_soc;
+    f.sparse = f.scalar ? ctx->d_ell_col != nullptr : ctx->sparse_local;
+    return f;
+}
 
-// Vectors a solve of nb bands carries: with the guard bands in mixed precision, whole Kramers pairs where
-// the matrix is quaternionic.
-int subspace(const uepm_ctx* ctx, int nb) {
-    if (ctx->precision != UEPM_PREC_MIXED) return nb;
-    const int m = std::min(ctx->n, nb + kGuardBands);
-    return quaternionic(ctx) ? (m + 1) & ~1 : m;
+// Bands a solve of nb bands computes: each scalar level is two of them.
+int form_bands(const Form& f, int nb) { return f.scalar ? (nb + 1) / 2 : nb; }
+// Vectors it carries: with the guard bands in mixed precision, whole Kramers pairs in quaternion form.
+int subspace(const uepm_ctx* ctx, const Form& f, int nb) {
+    const int nf = form_bands(f, nb);
+    if (ctx->precision != UEPM_PREC_MIXED) return nf;
+    const int m = std::min(f.n, nf + kGuardBands);
+    return f.quat ? (m + 1) & ~1 : m;
 }
 
 // Bytes of workspace one chunk of `c` matrices needs, with the offset of every region.
 Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
-    const size_t n = ctx->n, N = ctx->N;
+    const Form   f = form_of(ctx);
+    const size_t n = f.n, N = ctx->N;
     const bool   mixed = ctx->precision == UEPM_PREC_MIXED;
     const bool   vecs  = (want & (UEPM_WANT_VECTORS | UEPM_WANT_GRADIENT)) != 0;
-    const size_t m     = (size_t)subspace(ctx, nb);
-    const size_t es    = ctx->real ? sizeof(double) : sizeof(cx<double>);  // FP64 matrix scalar
-    const size_t es32  = ctx->real ? sizeof(float) : sizeof(cx<float>);   // FP32 matrix scalar
+    const size_t m     = (size_t)subspace(ctx, f, nb), nf = (size_t)form_bands(f, nb);
+    const size_t es    = f.real ? sizeof(double) : sizeof(cx<double>);  // FP64 matrix scalar
+    const size_t es32  = f.real ? sizeof(float) : sizeof(cx<float>);   // FP32 matrix scalar
     const size_t rs    = mixed ? sizeof(float) : sizeof(double);           // real type of the reduction
     Layout       L{};
     size_t       off = 0;
@@ -184,13 +206,13 @@ Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
         return o;
     };
     L.rows   = take(c * N * ROW_STRIDE * sizeof(double));
-    L.rows32 = (mixed && (ctx->ds_nl || ctx->ds_soc)) ? take(c * N * ROW_STRIDE * sizeof(float2)) : 0;
-    L.H    = take(mixed && ctx->sparse_local ? 0 : c * n * n * es);  // the sparse path never forms it
+    L.rows32 = (mixed && (f.ds_nl || f.ds_soc)) ? take(c * N * ROW_STRIDE * sizeof(float2)) : 0;
+    L.H    = take(mixed && f.sparse ? 0 : c * n * n * es);  // the sparse path never forms it
     L.H32  = mixed ? take(c * n * n * es32) : 0;
     L.d    = take(c * n * rs);
     L.e    = take(c * n * rs);
     L.tq   = take(c * n * (mixed ? es32 : es));
-    L.ev   = mixed || quaternionic(ctx) ? take(c * m * rs) : 0;
+    L.ev   = mixed || f.quat ? take(c * m * rs) : 0;
     if (mixed || vecs) {
         L.work = take(c * invit_work_elems<double>((int)n) * rs);
         L.z    = take(c * m * n * rs);
@@ -198,7 +220,12 @@ Layout plan(const uepm_ctx* ctx, int nb, uint32_t want, size_t c) {
     if (mixed) {
         L.X32    = take(c * m * n * sizeof(cx<float>));
         L.refine = take(c * refine_work_elems((int)n, (int)m) * es);
-        L.small  = take(c * refine_small_elems((int)m, nb) * es);
+        L.small  = take(c * refine_small_elems((int)m, (int)nf) * es);
+    }
+    if (f.scalar) {  // the scalar levels, vectors and gradients before they are written for both spins
+        L.fE = take(c * nf * sizeof(double));
+        if (want & UEPM_WANT_VECTORS) L.fX = take(c * nf * N * sizeof(cx<double>));
+        if (want & UEPM_WANT_GRADIENT) L.fg = take(c * nf * 3 * sizeof(double));
     }
     L.total = off;
     return L;
@@ -231,20 +258,21 @@ int check_launch() {
 // One chunk of c k-points through the pipeline, FP64 (S = double for real H, cx<double> otherwise)
 // or mixed precision (FP32 reduction in Lower<S>, FP64 Rayleigh-Ritz in S).
 template <typename S>
-void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c, int nb, int m, bool vec, double* E,
-               cx<double>* Xo, double* gr, int* st, cudaStream_t s) {
+void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const double* kk, int c, int nb, int m, bool vec,
+               double* E, cx<double>* Xo, double* gr, int* st, cudaStream_t s) {
     using S32            = typename Lower<S>::type;
-    const int    n       = ctx->n;
+    const int    n       = f.n;
     const size_t mstride = (size_t)n * n;
+    const DevParams& P   = f.scalar ? ctx->Ps : ctx->P;
     auto*        rows    = reinterpret_cast<double*>(ws + L.rows);
     auto*        H       = reinterpret_cast<S*>(ws + L.H);
-    const bool   ds_asm  = ctx->precision == UEPM_PREC_MIXED && (ctx->ds_nl || ctx->ds_soc);
+    const bool   ds_asm  = ctx->precision == UEPM_PREC_MIXED && (f.ds_nl || f.ds_soc);
     auto*        rows32  = ds_asm ? reinterpret_cast<float2*>(ws + L.rows32) : nullptr;
     {
         ProfScope p(ctx, s, KK_ROWS);
-        launch_rows(ctx->P, kk, ctx->d_G, rows, c, s, rows32);
+        launch_rows(P, kk, ctx->d_G, rows, c, s, rows32);
     }
-    const bool quat = quaternionic(ctx);
+    const bool quat = f.quat;
     const int  N = ctx->N, nz = (m + 1) / 2;  // quaternion order, pairs
     if (ctx->precision != UEPM_PREC_MIXED && quat) {
         if constexpr (ST<S>::cplx) {
@@ -256,7 +284,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
             auto*        ev = reinterpret_cast<double*>(ws + L.ev);
             {
                 ProfScope p(ctx, s, KK_ASSEMBLE);
-                launch_assemble_quat(ctx->P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, HQ, qs, c, s);
+                launch_assemble_quat(P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, HQ, qs, c, s);
             }
             {
                 ProfScope p(ctx, s, KK_TRIDIAG64);
@@ -275,7 +303,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
                     launch_invit<double>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
                 }
                 ProfScope p(ctx, s, KK_BACKTRANSFORM);
-                launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, ctx->P, kk, ctx->d_G, gr, c, s);
+                launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, P, kk, ctx->d_G, gr, c, s);
             }
         }
         return;
@@ -283,7 +311,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
     if (ctx->precision != UEPM_PREC_MIXED) {
         {
             ProfScope p(ctx, s, KK_ASSEMBLE);
-            launch_assemble<S>(ctx->P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, H, n, mstride, nullptr, 0, c, s);
+            launch_assemble<S>(P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, H, n, mstride, nullptr, 0, c, s);
         }
         auto* d  = reinterpret_cast<double*>(ws + L.d);
         auto* e  = reinterpret_cast<double*>(ws + L.e);
@@ -305,7 +333,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
                 launch_invit<double>(d, e, E, nb, n, nb, work, z, st, c, s, ctx->tune.max_iter);
             }
             ProfScope p(ctx, s, KK_BACKTRANSFORM);
-            launch_backtransform<S>(H, n, n, mstride, tq, z, nb, Xo, ctx->P, kk, ctx->d_G, gr, c, s, ctx->tune.vector_lanes);
+            launch_backtransform<S>(H, n, n, mstride, tq, z, nb, Xo, P, kk, ctx->d_G, gr, c, s, ctx->tune.vector_lanes);
         }
         return;
     }
@@ -315,24 +343,24 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
     // Real local-potential matrices reduced in registers: the reduction forms H(k) itself from the
     // resident V and the kinetic diagonal (the same FP32 values), so nothing is assembled.
     constexpr bool kReal32 = std::is_same<S32, float>::value;
-    const bool     reg_local = kReal32 && ctx->sparse_local && (ctx->tune.reduction == 0 || ctx->tune.reduction == 1) &&
+    const bool     reg_local = kReal32 && f.sparse && (ctx->tune.reduction == 0 || ctx->tune.reduction == 1) &&
                            n <= tridiag_reg_max_n();
     if (!reg_local) {
         ProfScope p(ctx, s, KK_ASSEMBLE);
         // the FP64 matrix is kept only for the Rayleigh-Ritz products: stored as FP32 pairs in place;
         // with a local potential only, those products use the resident sparse V instead
-        if (ctx->sparse_local)
-            launch_assemble<S32>(ctx->P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, H32, n, mstride, nullptr, 0, c, s);
-        else if (ds_asm && ctx->ds_soc) {
+        if (f.sparse)
+            launch_assemble<S32>(P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, H32, n, mstride, nullptr, 0, c, s);
+        else if (ds_asm && f.ds_soc) {
             if constexpr (std::is_same<SP, ds4>::value)
-                launch_assemble_soc_ds<SP>(ctx->P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, ctx->d_phSO32, rows32, ctx->d_Vloc,
+                launch_assemble_soc_ds<SP>(P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, ctx->d_phSO32, rows32, ctx->d_Vloc,
                                            ctx->d_phNL, ctx->d_phSO, rows, Hs, n, mstride, quat ? nullptr : H32, mstride, c,
                                            s, quat ? reinterpret_cast<qt<float>*>(H32) : nullptr, (size_t)N * N);
         } else if (ds_asm)
-            launch_assemble_ds<SP>(ctx->P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, rows32, ctx->d_Vloc, ctx->d_phNL, rows, Hs, n,
+            launch_assemble_ds<SP>(P, ctx->Q, ctx->d_Vloc32, ctx->d_phNL32, rows32, ctx->d_Vloc, ctx->d_phNL, rows, Hs, n,
                                    mstride, H32, mstride, c, s);
         else
-            launch_assemble<SP>(ctx->P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, Hs, n, mstride, H32, mstride, c, s);
+            launch_assemble<SP>(P, ctx->d_Vloc, ctx->d_phNL, ctx->d_phSO, rows, Hs, n, mstride, H32, mstride, c, s);
     }
     auto* d     = reinterpret_cast<float*>(ws + L.d);
     auto* e     = reinterpret_cast<float*>(ws + L.e);
@@ -362,7 +390,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
             launch_invit<float>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
         }
         ProfScope p(ctx, s, KK_BACKTRANSFORM);
-        launch_backtransform_quat<float>(HQ, N, N, qs, qq, z, nz, m, X32, ctx->P, kk, ctx->d_G, nullptr, c, s);
+        launch_backtransform_quat<float>(HQ, N, N, qs, qq, z, nz, m, X32, P, kk, ctx->d_G, nullptr, c, s);
     } else {
     {
         ProfScope p(ctx, s, KK_TRIDIAG32);
@@ -387,13 +415,13 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
     }
     {
         ProfScope p(ctx, s, KK_BACKTRANSFORM);
-        launch_backtransform<S32>(H32, n, n, mstride, tq, z, m, X32, ctx->P, kk, ctx->d_G, nullptr, c, s,
+        launch_backtransform<S32>(H32, n, n, mstride, tq, z, m, X32, P, kk, ctx->d_G, nullptr, c, s,
                                   ctx->tune.vector_lanes);
     }
     }
     {
         ProfScope p(ctx, s, KK_REFINE_PROJECT);
-        const SparseV sv{ctx->sparse_local, ctx->ell_w,  ctx->d_ell_col, ctx->d_ell_re,
+        const SparseV sv{f.sparse, ctx->ell_w,  ctx->d_ell_col, ctx->d_ell_re,
                          ctx->d_ell_im,       ctx->d_Vloc, rows,            ctx->N};
         launch_refine_project<S>(Hs, n, n, mstride, X32, m, rw, small, c, s, sv, st, ctx->tune.tensor_cores == 0,
                                  quat ? N : 0);
@@ -405,7 +433,7 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
     }
     if (vec) {
         ProfScope p(ctx, s, KK_REFINE_VECTORS);
-        launch_refine_vectors<S>(n, m, nb, X32, W, Xo, gr, ctx->P, kk, ctx->d_G, c, s);
+        launch_refine_vectors<S>(n, m, nb, X32, W, Xo, gr, P, kk, ctx->d_G, c, s);
     }
 }
 
@@ -414,6 +442,15 @@ void run_chunk(uepm_ctx* ctx, const Layout& L, char* ws, const double* kk, int c
 namespace uepm {
 
 int ensure_workspace(uepm_ctx* ctx, size_t bytes) { return ensure_ws(ctx, bytes); }
+
+double reduction_cost(const uepm_ctx* ctx) {
+    const Form   f = form_of(ctx);
+    const double N = f.quat ? ctx->N : f.n;
+    return N * N * N * (f.quat ? 16.0 : f.real ? 1.0 : 4.0);
+}
+int solve_form(const uepm_ctx* ctx) {
+    return ctx->force_cx ? 0 : ctx->decoupled ? (ctx->scalar_real ? 3 : 1) : ctx->quat_h ? 2 : 0;
+}
 
 // Two lanes: a mixed solve's reduction holds the SMs' registers or shared memory, and the kernels
 // after it (bisection, inverse iteration, the Rayleigh-Ritz products and the small solves) are bound
@@ -434,9 +471,8 @@ int plan_solve(uepm_ctx* ctx, size_t nk, int nb, uint32_t want, SolvePlan* out, 
         return UEPM_ERR_OUT_OF_RANGE;
     }
     const bool mixed = ctx->precision == UEPM_PREC_MIXED;
-    const int  n     = ctx->n;
-    const int  m     = subspace(ctx, nb);
-    if (mixed && m > kRefineMaxSubspace) {
+    const int  m     = subspace(ctx, form_of(ctx), nb);
+    if (mixed && std::min(ctx->n, nb + kGuardBands) > kRefineMaxSubspace) {
         set_error("mixed precision supports at most " + std::to_string(kRefineMaxSubspace - kGuardBands) + " bands");
         return UEPM_ERR_INVALID;
     }
@@ -468,6 +504,7 @@ int enqueue_solve(uepm_ctx* ctx, const SolvePlan& sp, const double* d_k, size_t 
     }
     const int    n     = ctx->n;
     const size_t chunk = sp.chunk;
+    const Form   f     = form_of(ctx);
     const Layout L     = plan(ctx, nb, want, chunk);
     char*        ws    = static_cast<char*>(ws_ext ? ws_ext : ctx->d_ws);
     if (d_status) UEPM_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int32_t) * nk, s));
@@ -510,8 +547,18 @@ int enqueue_solve(uepm_ctx* ctx, const SolvePlan& sp, const double* d_k, size_t 
         double*       E  = d_E + off * nb;
         cx<double>*   Xo = want_vec ? reinterpret_cast<cx<double>*>(d_X) + off * nb * n : nullptr;
         double*       gr = want_grad ? d_grad + off * nb * 3 : nullptr;
-        if (ctx->real) run_chunk<double>(ctx, L, wsq, kk, c, nb, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
-        else run_chunk<cx<double>>(ctx, L, wsq, kk, c, nb, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
+        if (f.scalar) {
+            E  = reinterpret_cast<double*>(wsq + L.fE);
+            Xo = want_vec ? reinterpret_cast<cx<double>*>(wsq + L.fX) : nullptr;
+            gr = want_grad ? reinterpret_cast<double*>(wsq + L.fg) : nullptr;
+        }
+        const int nf = form_bands(f, nb);
+        if (f.real) run_chunk<double>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
+        else run_chunk<cx<double>>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
+        if (f.scalar)
+            launch_spin_pairs(E, Xo, gr, ctx->N, nf, nb, c, d_E + off * nb,
+                              want_vec ? reinterpret_cast<cx<double>*>(d_X) + off * nb * n : nullptr,
+                              want_grad ? d_grad + off * nb * 3 : nullptr, sq);
         if ((rc = check_launch())) break;
     }
     if (forked) {  // join (also after a failed launch): work enqueued on s later waits for the second lane
@@ -567,6 +614,11 @@ int uepm_ctx_create(const uepm_material* mat, const int32_t* G, int N, uint32_t 
     ctx->quat_h = soc && mat->V3A == 0.0 && mat->V4A == 0.0 && mat->V8A == 0.0 && mat->V11A == 0.0 && same_nl &&
                   (mat->mu_soc == 0.0 || (mat->period_anion == mat->period_cation && mat->alpha_soc == 1.0 &&
                                           mat->radial_extent_anion == mat->radial_extent_cation));
+    // No spin-orbit strength: the spin-orbit blocks vanish identically, H = diag(h, h)
+    ctx->decoupled   = soc && mat->mu_soc == 0.0 && std::isfinite(mat->alpha_soc) && std::isfinite(mat->radial_extent_anion) &&
+                     std::isfinite(mat->radial_extent_cation) && mat->radial_extent_anion != 0.0 &&
+                     mat->radial_extent_cation != 0.0;
+    ctx->scalar_real = ctx->decoupled && mat->V3A == 0.0 && mat->V4A == 0.0 && mat->V8A == 0.0 && mat->V11A == 0.0 && same_nl;
     cudaGetDevice(&ctx->device);
 
     // Derived constants, each with the reference's own expression.
@@ -664,8 +716,13 @@ int uepm_ctx_create(const uepm_material* mat, const int32_t* G, int N, uint32_t 
         if ((e = cudaMemcpy(ctx->d_phNL, phNL.data(), sizeof(double2) * phNL.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e, "copy phNL");
     }
-    ctx->ds_nl  = nl && !soc && (P.has_R0a || P.has_R0c || P.has_A2a || P.has_A2c);
-    ctx->ds_soc = soc;
+    const bool wells  = nl && (P.has_R0a || P.has_R0c || P.has_A2a || P.has_A2c);
+    ctx->ds_nl        = wells && !soc;
+    ctx->ds_soc       = soc;
+    ctx->scalar_ds_nl = wells && ctx->decoupled;
+    ctx->Ps           = P;
+    ctx->Ps.soc       = 0;
+    ctx->Ps.n         = N;
     if (ctx->ds_nl || ctx->ds_soc) {
         // the nonlocal constants and the k-independent tables as FP32 pairs; products the FP64
         // element forms first are formed here in FP64, in the same order
@@ -722,7 +779,7 @@ int uepm_ctx_create(const uepm_material* mat, const int32_t* G, int N, uint32_t 
         if ((e = cudaMemcpy(ctx->d_phSO, phSO.data(), sizeof(double2) * phSO.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e, "copy phSO");
     }
-    if (!nl && !soc) {
+    if (!nl && (!soc || ctx->decoupled)) {
         // V off the diagonal in transposed ELL form (slot e of row i at [e][i], columns ascending
         // within a row, short rows padded with zero values at column i); values split into FP32
         // pairs (round to nearest, as on the device). The diagonal gets the kinetic term per k on
@@ -772,7 +829,7 @@ int uepm_ctx_create(const uepm_material* mat, const int32_t* G, int N, uint32_t 
         if ((e = cudaMalloc(&ctx->d_V32, sizeof(float) * v32.size())) != cudaSuccess) return fail(e, "cudaMalloc(V32)");
         if ((e = cudaMemcpy(ctx->d_V32, v32.data(), sizeof(float) * v32.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e, "copy V32");
-        ctx->sparse_local = true;
+        ctx->sparse_local = !soc;
     }
     *out = ctx;
     return UEPM_OK;

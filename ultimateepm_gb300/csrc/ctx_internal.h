@@ -23,6 +23,9 @@ struct uepm_ctx {
     // H(k) of a spin-orbit context is quaternionic: time reversal times inversion is a symmetry at every
     // k (no antisymmetric form factors, equal atoms), so every level is a Kramers pair
     bool          quat_h    = false;
+    // a spin-orbit context without spin-orbit strength, H = diag(h, h): solved on h (Ps: P of the scalar problem)
+    bool          decoupled = false, scalar_real = false, scalar_ds_nl = false;
+    uepm::DevParams Ps{};
     size_t        ws_limit  = (size_t)8 << 30;
     uepm_tuning   tune{};  // kernel-shape choices (0: automatic)
     int*          d_G       = nullptr;
@@ -95,6 +98,11 @@ int ensure_workspace(uepm_ctx* ctx, size_t bytes);
 int enqueue_solve(uepm_ctx* ctx, const SolvePlan& plan, const double* d_k, size_t nk, int nb, uint32_t want, double* d_E,
                   double* d_X, double* d_grad, int32_t* d_status, cudaStream_t s, void* ws = nullptr,
                   size_t ws_bytes = 0);
+// Multiply-adds of one matrix's reduction, up to a common factor: what groups are ordered by.
+double reduction_cost(const uepm_ctx* ctx);
+// The form that an automatic solve of the context works on (0: the matrix itself, 1 or 3: complex or real scalar,
+// 2: quaternion): part of the key under which tunings are shared.
+int solve_form(const uepm_ctx* ctx);
 uint64_t launches_total();
 void     uncount_launches(uint64_t n);
 

@@ -120,6 +120,10 @@ template <typename T>
 void launch_backtransform_quat(const qt<T>* H, int n, int ld, size_t mstride, const qt<T>* tq, const T* z, int nz, int nb,
                                cx<T>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
                                int batch, cudaStream_t s);
+// The nf scalar levels, vectors ([batch][nf][N]) and gradients of H = diag(h, h) as nb bands for both spins:
+// band 2 q is level q with spin up (x, 0), band 2 q + 1 with spin down (0, x). X, g and their outputs may be null.
+void launch_spin_pairs(const double* E, const cx<double>* X, const double* g, int N, int nf, int nb, int batch, double* Eo,
+                       cx<double>* Xo, double* go, cudaStream_t s);
 // E[b][i] = ev[b][i / 2], i < nb: the doubly degenerate values of a quaternion matrix (backtransform.cu)
 void launch_pair_values(const double* ev, int nz, double* E, int nb, int batch, cudaStream_t s);
 
