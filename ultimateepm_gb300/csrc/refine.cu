@@ -77,27 +77,68 @@ __device__ __forceinline__ typename Split<S>::type sparse_slot(const SparseV& sv
     }
 }
 
-// y[q] += h x(c, j0 + q), q < kProjVB
+// The vectors' values at row c: kProjVB of them, packed as the accumulators are (real: vectors in pairs;
+// complex: each vector's real and imaginary part).
 template <typename S, bool STAGED>
-__device__ __forceinline__ void proj_accumulate(dsacc (&yr)[kProjVB], dsacc (&yi)[kProjVB], const typename Split<S>::type& h,
-                                                const XElem<S>* Xs, const cx<float>* Xg, int n, int m, int mp, int c,
-                                                int j0) {
+__device__ __forceinline__ void x_block(const XElem<S>* Xs, const cx<float>* Xg, int n, int m, int mp, int c, int j0,
+                                        float (&x)[kProjVB * sizeof(XElem<S>) / 4]) {
+    constexpr int V = kProjVB * sizeof(XElem<S>) / 4;
+    if constexpr (STAGED) {
+        const float4* src = reinterpret_cast<const float4*>(Xs + (size_t)c * mp + j0);  // mp and j0 are multiples of 4
 #pragma unroll
-    for (int q = 0; q < kProjVB; ++q) {
-        const XElem<S> x = x_at<S, STAGED>(Xs, Xg, n, m, mp, c, j0 + q);
-        if constexpr (!std::is_same<S, double>::value) {  // (hr + i hi)(xr + i xi)
-            ds_add_prod(yr[q], h.rhi, h.rlo, x.x);
-            ds_add_prod(yr[q], -h.ihi, -h.ilo, x.y);
-            ds_add_prod(yi[q], h.rhi, h.rlo, x.y);
-            ds_add_prod(yi[q], h.ihi, h.ilo, x.x);
-        } else {
-            ds_add_prod(yr[q], h.hi, h.lo, x);
+        for (int q = 0; q < V / 4; ++q) {
+            const float4 v = src[q];
+            x[4 * q]       = v.x;
+            x[4 * q + 1]   = v.y;
+            x[4 * q + 2]   = v.z;
+            x[4 * q + 3]   = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < kProjVB; ++q) {
+            const XElem<S> v = x_at<S, false>(Xs, Xg, n, m, mp, c, j0 + q);
+            if constexpr (V == 2 * kProjVB) {
+                x[2 * q]     = v.x;
+                x[2 * q + 1] = v.y;
+            } else {
+                x[q] = v;
+            }
         }
     }
 }
 
+// y += h x(c, j0 ..) for the kProjVB vectors: y[q] holds vectors 2 q and 2 q + 1 (real) or vector q's parts (complex).
+// Two accumulations per instruction (the scalar form was bound by issue and, per column, by the latency of H).
+template <typename S, bool STAGED>
+__device__ __forceinline__ void proj_accumulate(dsacc2* y, const typename Split<S>::type& h, const XElem<S>* Xs,
+                                                const cx<float>* Xg, int n, int m, int mp, int c, int j0) {
+    constexpr bool CX = !std::is_same<S, double>::value;
+    float          x[kProjVB * sizeof(XElem<S>) / 4];
+    x_block<S, STAGED>(Xs, Xg, n, m, mp, c, j0, x);
+    if constexpr (CX) {  // (hr + i hi)(xr + i xi)
+        const f32x2 rh = pack2(h.rhi, h.rhi), nrh = pack2(-h.rhi, -h.rhi), rl = pack2(h.rlo, h.rlo);
+        const f32x2 ih = pack2(-h.ihi, h.ihi), nih = pack2(h.ihi, -h.ihi), il = pack2(-h.ilo, h.ilo);
+#pragma unroll
+        for (int q = 0; q < kProjVB; ++q) {
+            ds_add_prod(y[q], rh, nrh, rl, pack2(x[2 * q], x[2 * q + 1]));
+            ds_add_prod(y[q], ih, nih, il, pack2(x[2 * q + 1], x[2 * q]));
+        }
+    } else {
+        const f32x2 hh = pack2(h.hi, h.hi), nh = pack2(-h.hi, -h.hi), hl = pack2(h.lo, h.lo);
+#pragma unroll
+        for (int q = 0; q < kProjVB / 2; ++q) ds_add_prod(y[q], hh, nh, hl, pack2(x[2 * q], x[2 * q + 1]));
+    }
+}
+
+// CTAs per SM that the registers must allow: more loads in flight per thread against more threads
+template <typename S, bool SPARSE, bool YDONE>
+constexpr int proj_min_blocks() {
+    if (std::is_same<S, double>::value) return SPARSE ? 1 : 4;
+    return YDONE ? 4 : 3;
+}
+
 template <typename S, bool STAGED, bool SPARSE, bool YDONE = false>
-__global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split<S>::type* __restrict__ H, int n, int ld,
+__global__ void __launch_bounds__(kProjNT, proj_min_blocks<S, SPARSE, YDONE>()) k_refine_project(const typename Split<S>::type* __restrict__ H, int n, int ld,
                                                             size_t mstride, const cx<float>* __restrict__ X32, int m,
                                                             void* __restrict__ work, S* __restrict__ small, int batch,
                                                             const SparseV sv, int nr) {
@@ -114,7 +155,7 @@ __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split
     if (STAGED) {
         // asynchronous element copies (all in flight at once); the padding vectors j >= m are zero
         const int warp = tid >> 5, lane = tid & 31;
-        for (int j = warp; j < mp; j += kProjNT / 32) {
+        for (int j = warp; j < mp; j += blockDim.x / 32) {
             for (int r = lane; r < n; r += 32) {
                 XT* dst = Xs + (size_t)r * mp + j;
                 if (j < m) cp_async_elem<sizeof(XT)>(dst, Xg + (size_t)j * n + r);  // Re, or (Re, Im)
@@ -133,37 +174,57 @@ __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split
     // nr < n: a quaternionic H, of which only the first nr = n / 2 rows exist; the vectors are pairs, and the
     // rows below follow from the pair's other member (Y(r + nr, 2 p) = -conj Y(r, 2 p + 1), Y(r + nr, 2 p + 1) =
     // conj Y(r, 2 p))
-    for (int item = tid; item < (YDONE ? 0 : nblk * nr); item += kProjNT) {  // YDONE: Y came from the tensor cores
-        const int r = item / nblk, jb = item - r * nblk, j0 = jb * kProjVB;
-        dsacc     yr[kProjVB], yi[kProjVB];
+    for (int item = tid; item < (YDONE ? 0 : nblk * nr); item += blockDim.x) {  // YDONE: Y came from the tensor cores
+        const int     r = item / nblk, jb = item - r * nblk, j0 = jb * kProjVB;
+        constexpr int NA = CX ? kProjVB : kProjVB / 2;
+        dsacc2        y[NA];
 #pragma unroll
-        for (int q = 0; q < kProjVB; ++q) yr[q] = yi[q] = dsacc{0.f, 0.f};
+        for (int q = 0; q < NA; ++q) y[q] = dsacc2{0ull, 0ull};
         if constexpr (SPARSE) {
             // the diagonal, then the off-diagonal slots (coalesced over r)
-            proj_accumulate<S, STAGED>(yr, yi, sparse_diag<S>(sv, b, r), Xs, Xg, n, m, mp, r, j0);
+            proj_accumulate<S, STAGED>(y, sparse_diag<S>(sv, b, r), Xs, Xg, n, m, mp, r, j0);
 #pragma unroll 4
             for (int e = 0; e < sv.W; ++e) {
                 const size_t o = (size_t)e * sv.N + r;
-                proj_accumulate<S, STAGED>(yr, yi, sparse_slot<S>(sv, o), Xs, Xg, n, m, mp, sv.col[o], j0);
+                proj_accumulate<S, STAGED>(y, sparse_slot<S>(sv, o), Xs, Xg, n, m, mp, sv.col[o], j0);
             }
         } else {
-            SE h = A[r];
-            for (int c = 0; c < n; ++c) {
-                const SE hc = h;
-                if (c + 1 < n) h = A[(size_t)(c + 1) * ld + r];
-                proj_accumulate<S, STAGED>(yr, yi, hc, Xs, Xg, n, m, mp, c, j0);
-            }
-        }
+            // kAhead columns of H in flight: an element's latency (HBM, mostly: the reduction ran in between) is longer
+            // than one column's products of the warps that share a scheduler. 20000 k of Si nonlocal (n = 137 real)
+            // 5.09 -> 2.96 ms with the packed sums, 10007 k of Ge (181) 3.88 -> 2.36, 20011 k of InP (113, complex)
+            // 7.89 -> 7.14 (4.5 ms at the FP32 pipe's rate).
+            constexpr int kAhead = CX ? 4 : 8;
+            SE            h[kAhead];
 #pragma unroll
-        for (int q = 0; q < kProjVB; ++q) {
-            if constexpr (CX) {
-                Y[(size_t)r * mp + j0 + q] = make_float4(yr[q].h, yr[q].l, yi[q].h, yi[q].l);
-                if (nr < n) {
-                    const float sg = q & 1 ? -1.f : 1.f;
-                    Y[(size_t)(r + nr) * mp + j0 + (q ^ 1)] = make_float4(sg * yr[q].h, sg * yr[q].l, -sg * yi[q].h, -sg * yi[q].l);
+            for (int q = 0; q < kAhead; ++q) h[q] = A[(size_t)min(q, n - 1) * ld + r];
+            int c = 0;
+            for (; c + kAhead <= n; c += kAhead) {
+#pragma unroll
+                for (int q = 0; q < kAhead; ++q) {
+                    const SE hc = h[q];
+                    h[q]        = A[(size_t)min(c + q + kAhead, n - 1) * ld + r];
+                    proj_accumulate<S, STAGED>(y, hc, Xs, Xg, n, m, mp, c + q, j0);
                 }
             }
-            else Y[(size_t)r * mp + j0 + q] = make_float2(yr[q].h, yr[q].l);
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q)
+                if (c + q < n) proj_accumulate<S, STAGED>(y, h[q], Xs, Xg, n, m, mp, c + q, j0);
+        }
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+            float h0, h1, l0, l1;
+            unpack2(y[q].h, h0, h1);
+            unpack2(y[q].l, l0, l1);
+            if constexpr (CX) {
+                Y[(size_t)r * mp + j0 + q] = make_float4(h0, l0, h1, l1);
+                if (nr < n) {
+                    const float sg = q & 1 ? -1.f : 1.f;
+                    Y[(size_t)(r + nr) * mp + j0 + (q ^ 1)] = make_float4(sg * h0, sg * l0, -sg * h1, -sg * l1);
+                }
+            } else {
+                Y[(size_t)r * mp + j0 + 2 * q]     = make_float2(h0, l0);
+                Y[(size_t)r * mp + j0 + 2 * q + 1] = make_float2(h1, l1);
+            }
         }
     }
     __syncthreads();
@@ -171,31 +232,38 @@ __global__ void __launch_bounds__(kProjNT) k_refine_project(const typename Split
     S*        Sg = small + (size_t)b * refine_small_elems(m, 0);
     S*        Ag = Sg + (size_t)m * m;
     const int np = m * (m + 1) / 2;
-    for (int k = tid; k < np; k += kProjNT) {
+    for (int k = tid; k < np; k += blockDim.x) {
         int p = 0, rest = k;
         while (rest >= m - p) {
             rest -= m - p;
             ++p;
         }
         const int q = p + rest;
-        dsacc     sr{0.f, 0.f}, si{0.f, 0.f}, ar{0.f, 0.f}, ai{0.f, 0.f};
+        dsacc2    s2{0ull, 0ull}, a2{0ull, 0ull};  // complex: S and A's parts; real: (S, A) in s2
+#pragma unroll (CX ? 2 : 4)
         for (int r = 0; r < n; ++r) {
             const XT xp = x_at<S, STAGED>(Xs, Xg, n, m, mp, r, p);
             const XT xq = x_at<S, STAGED>(Xs, Xg, n, m, mp, r, q);
             const YT y  = Y[(size_t)r * mp + q];
             if constexpr (CX) {  // conj(xp) xq and conj(xp) y
-                ds_add_prod(sr, xp.x, xq.x);
-                ds_add_prod(sr, xp.y, xq.y);
-                ds_add_prod(si, xp.x, xq.y);
-                ds_add_prod(si, -xp.y, xq.x);
-                ds_add_prod(ar, y.x, y.y, xp.x);
-                ds_add_prod(ar, y.z, y.w, xp.y);
-                ds_add_prod(ai, y.z, y.w, xp.x);
-                ds_add_prod(ai, -y.x, -y.y, xp.y);
+                const f32x2 xr = pack2(xp.x, xp.x), xi = pack2(xp.y, xp.y), zero = 0ull;
+                ds_add_prod(s2, pack2(xq.x, xq.y), pack2(-xq.x, -xq.y), zero, xr);
+                ds_add_prod(s2, pack2(xq.y, -xq.x), pack2(-xq.y, xq.x), zero, xi);
+                ds_add_prod(a2, pack2(y.x, y.z), pack2(-y.x, -y.z), pack2(y.y, y.w), xr);
+                ds_add_prod(a2, pack2(y.z, -y.x), pack2(-y.z, y.x), pack2(y.w, -y.y), xi);
             } else {
-                ds_add_prod(sr, xp, xq);
-                ds_add_prod(ar, y.x, y.y, xp);
+                ds_add_prod(s2, pack2(xq, y.x), pack2(-xq, -y.x), pack2(0.f, y.y), pack2(xp, xp));
             }
+        }
+        dsacc sr, si{0.f, 0.f}, ar, ai{0.f, 0.f};
+        if constexpr (CX) {
+            unpack2(s2.h, sr.h, si.h);
+            unpack2(s2.l, sr.l, si.l);
+            unpack2(a2.h, ar.h, ai.h);
+            unpack2(a2.l, ar.l, ai.l);
+        } else {
+            unpack2(s2.h, sr.h, ar.h);
+            unpack2(s2.l, sr.l, ar.l);
         }
         const S s = ST<S>::make(ds_value(sr), ds_value(si)), a = ST<S>::make(ds_value(ar), ds_value(ai));
         Sg[p * m + q] = s;
@@ -666,12 +734,15 @@ static void refine_project_t(const typename Split<S>::type* H, int n, int ld, si
                              S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int half = 0) {
     const int    nr    = half ? half : n;
     const size_t stage = proj_stage_bytes<S>(n, m);
+    // as many threads as leave few idle in the last round of Y's work items
+    const int items = YDONE ? 0 : nr * (proj_mp<S>(m) / kProjVB), rounds = (items + kProjNT - 1) / kProjNT;
+    const int nt = rounds ? (items + 32 * rounds - 1) / (32 * rounds) * 32 : kProjNT;
     if (stage <= kProjStageBytes) {
         auto kern = k_refine_project<S, true, SPARSE, YDONE>;
         if (stage > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage);
-        kern<<<batch, kProjNT, stage, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
+        kern<<<batch, nt, stage, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
     } else {
-        k_refine_project<S, false, SPARSE, YDONE><<<batch, kProjNT, 0, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
+        k_refine_project<S, false, SPARSE, YDONE><<<batch, nt, 0, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
     }
     count_launch();
 }

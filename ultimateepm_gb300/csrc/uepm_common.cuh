@@ -371,6 +371,49 @@ __device__ __forceinline__ void ds_add_prod(dsacc& a, float x, float y) {
 }
 __device__ __forceinline__ double ds_value(dsacc a) { return (double)a.h + (double)a.l; }
 
+// Pairs of FP32 values in one 64-bit register pair (PTX's .f32x2 operations): two accumulations in the issue
+// slots of one, each operation rounded as its scalar form, so the sums are the same bits.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+struct dsacc2 {
+    f32x2 h, l;
+};
+// a += (xh + xl) y for both members; nxh = -xh
+__device__ __forceinline__ void ds_add_prod(dsacc2& a, f32x2 xh, f32x2 nxh, f32x2 xl, f32x2 y) {
+    const f32x2 p   = mul2(xh, y);
+    const f32x2 npe = fma2(nxh, y, p);  // minus the product's rounding error
+    const f32x2 s   = add2(a.h, p);
+    const f32x2 z   = sub2(s, a.h);
+    const f32x2 er  = add2(sub2(a.h, sub2(s, z)), sub2(p, z));
+    a.h             = s;
+    a.l             = fma2(xl, y, add2(a.l, sub2(er, npe)));
+}
+
 // Double-single numbers (an FP32 pair h + l, |l| <= ulp(h) / 2, about 48 significant bits) with the
 // classical error-free transformations (Dekker, Knuth) on non-contracted FP32 operations: the mixed
 // path evaluates the nonlocal matrix elements on the FP32 pipe with them instead of the FP64 pipe.
