@@ -130,7 +130,8 @@ void launch_pair_values(const double* ev, int nz, double* E, int nb, int batch, 
 // refine.cu: FP64 Rayleigh-Ritz in the m-dimensional subspace of FP32 vectors X32 ([batch][m][n]);
 // the nb lowest Ritz values go to Eout, optionally vectors / gradients.
 constexpr int kRefineMaxSubspace = 40;
-__host__ __device__ inline size_t refine_work_elems(int n, int m) { return (size_t)2 * n * m; }
+// Y's vectors are padded to a multiple of four, which 2 m covers but for m = 1
+__host__ __device__ inline size_t refine_work_elems(int n, int m) { return (size_t)n * (m > 1 ? 2 * m : 4); }
 // small-solve scratch per matrix, contiguous: S (m x m), A (m x m), then the m x nb (<= m x m) Ritz
 // coefficients W at offset 2 m^2
 __host__ __device__ inline size_t refine_small_elems(int m, int) { return (size_t)3 * m * m; }
