@@ -550,13 +550,19 @@ void launch_tridiag_quat(qt<double>* H, int n, int ld, size_t mstride, double* d
 template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant, int ctas_per_sm, int cluster, bool tensor_cores) {
-    // complex orders whose lower triangle fits one SM's shared memory and fills it alone: reduction of 1500
-    // matrices in ms, triangular against deferred (5) and blocked (6): n = 178 6.69, 7.45, 8.81; 181 6.76,
-    // 7.78, 8.97; 226 11.06, 13.92, 12.86; 229 11.97, 14.38, 13.11. Below, several deferred CTAs per SM hide
-    // more of the serial chain (2000 matrices, n = 113 3.02 against 2.37, 169 8.74 against 8.15).
-    if constexpr (std::is_same<S, cx<float>>::value)
+    // complex orders: registers to 144 (2000 matrices, n = 113 1.27 ms against 2.37 for the deferred kernel, 137 1.98
+    // against 3.78), then the deferred kernel (n = 169 8.15 against 8.74 for the triangular one), and the triangular
+    // kernel where the lower triangle fits one SM's shared memory and fills it alone (1500 matrices in ms, triangular
+    // against deferred (5) and blocked (6): n = 178 6.69, 7.45, 8.81; 181 6.76, 7.78, 8.97; 226 11.06, 13.92, 12.86;
+    // 229 11.97, 14.38, 13.11)
+    if constexpr (std::is_same<S, cx<float>>::value) {
+        if (variant == 0 && n <= tridiag_reg_max_n(true)) {
+            launch_tridiag_reg(H, n, ld, mstride, d, e, tq, status, batch, s);
+            return;
+        }
         if (variant == 0 && n >= 175 && n <= 230 && launch_tridiag_tri<S>(H, n, ld, mstride, d, e, tq, status, batch, s))
             return;
+    }
     if constexpr (std::is_same<S, float>::value) {
         if ((variant == 0 || variant == 1) && n <= tridiag_reg_max_n()) {
             launch_tridiag_reg(H, n, ld, mstride, d, e, tq, status, batch, s);
@@ -582,9 +588,7 @@ void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, t
             launch_tridiag_blocked<S>(H, n, ld, mstride, d, e, tq, status, batch, s, tensor_cores))
             return;
         // automatic: the deferred kernel for every FP32 order beyond the register kernel, also where
-        // the matrix would fit shared memory (2000 k: Ge nonlocal n = 181 real 5.85 ms against 14.3
-        // for the shared-memory kernel; InP n = 113 complex 2.37 against 3.27; GaAs n = 89 complex
-        // 1.45 against 1.70)
+        // the matrix would fit shared memory (2000 k: InP n = 169 complex 8.15 ms)
         const bool auto_fused = variant == 0;
         if (variant == 4 && n <= 512) {
             if (n <= 129) fused_launch_t<S, 4>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);

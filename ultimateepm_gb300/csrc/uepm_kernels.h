@@ -81,11 +81,13 @@ bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>:
 template <typename S>
 bool launch_tridiag_tri(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, int* status, int batch,
                         cudaStream_t s);
-// tridiag_reg.cu: the same reduction for real FP32 matrices with n <= tridiag_reg_max_n(), held in
-// registers (launch_tridiag<float> dispatches to it).
-int  tridiag_reg_max_n();
+// tridiag_reg.cu: the same reduction for FP32 matrices with n <= tridiag_reg_max_n(complex), held in
+// registers (launch_tridiag dispatches to it; complex ones in the automatic choice only).
+int  tridiag_reg_max_n(bool cplx = false);
 void launch_tridiag_reg(float* H, int n, int ld, size_t mstride, float* d, float* e, float* tq, int* status, int batch,
                         cudaStream_t s);
+void launch_tridiag_reg(cx<float>* H, int n, int ld, size_t mstride, float* d, float* e, cx<float>* tq, int* status,
+                        int batch, cudaStream_t s);
 // The same for real local-potential matrices formed in the kernel from the k-independent local V
 // ([N][N], N = n: its FP32 rounding V32 off the diagonal, FP64 Vloc plus the rows table's kinetic term
 // on it), bit-identical to reducing the assembly's FP32 copy; H receives only the reflector tails.
