@@ -374,16 +374,18 @@ __device__ __forceinline__ ds i2_ds(ds x) {
 // i2 of the gaussian well with radius R: x = R^2 / 2 n1 n2, from the FP64 norms where x <= 2 (the
 // FP64 element's own operands and function), else in double-single (R2h = R^2 / 2 as a pair, np =
 // n1 n2 in double-single).
-__device__ __forceinline__ ds i2_gauss(double R, ds R2h, ds np, double n1d, double n2d) {
+__device__ __forceinline__ ds i2_gauss(double R, ds R2h, ds np, const double& n1d, const double& n2d) {
+    const ds x = ds_mul(R2h, np);
+    if (x.h > 2.001f) return i2_ds(x);  // beyond 2 with any rounding
     const double argd = 0.5 * (R * R) * n1d * n2d;
-    return argd <= 2.0 ? ds_of_double(bessel_i2(argd)) : i2_ds(ds_mul(R2h, np));
+    return argd <= 2.0 ? ds_of_double(bessel_i2(argd)) : i2_ds(x);
 }
 
 // far: the reference's branch |n1 - n2| > 1e-4, decided on the FP64 norms by the caller (the
 // double-single difference is not resolved finely enough for it).
 // n1d, n2d: the FP64 norms (the gaussian well's argument at x <= 2, as the FP64 element forms it).
 __device__ void nl_element_ds(const DevParams& P, const DevParamsDS& Q, RowDS Ri, RowDS Rj, ds pc, ds ps,
-                              bool far, double n1d, double n2d, ds& re, ds& im) {
+                              bool far, const double& n1d, const double& n2d, ds& re, ds& im) {
     const ds   n1  = rd(Ri, RF_NK), n2 = rd(Rj, RF_NK);
     const ds   dp  = ds_add(ds_add(ds_mul(rd(Ri, RF_KX), rd(Rj, RF_KX)), ds_mul(rd(Ri, RF_KY), rd(Rj, RF_KY))),
                             ds_mul(rd(Ri, RF_KZ), rd(Rj, RF_KZ)));
@@ -571,19 +573,37 @@ __global__ void __launch_bounds__(256) k_assemble_tiles(const DevParams P, const
     }
 }
 
+// The FP64 tests of nl_needs_fp64: bit 0 far, bit 1 that the FP64 element is needed; Ra, Rc the gaussian wells' radii
+// or 0. A call, because a branch this short would be predicated, and FP64 instructions take the pipe even so.
+__device__ __noinline__ int nl_exact_tests(double n1, double n2, double Ra, double Rc) {
+    const double dn  = fabs(n1 - n2);
+    const bool   far = F_l_far(n1, n2);
+    const bool   need = (far && dn < 1.0e-5 * fmax(n1, n2)) || 0.5 * (Ra * Ra) * (n1 * n2) > 80.0 || 0.5 * (Rc * Rc) * (n1 * n2) > 80.0;
+    return (far ? 1 : 0) | (need ? 2 : 0);
+}
+
 // Whether the double-single nonlocal element must give way to the FP64 one for the pair of norms
 // (n1, n2): where the reference's far branch divides rounding-level differences (|n1 - n2| within
 // 1e-5 of the norms), and for gaussian wells where i2's argument x exceeds 80 (e^x beyond FP32's
 // range). far returns the reference's branch.
-__device__ __forceinline__ bool nl_needs_fp64(const DevParams& P, double n1, double n2, bool& far) {
-    const double dn = fabs(n1 - n2);
-    far             = F_l_far(n1, n2);
-    if (far && dn < 1.0e-5 * fmax(n1, n2)) return true;
-    if (!P.square) {
-        if (P.has_A2a && 0.5 * (P.R2a * P.R2a) * (n1 * n2) > 80.0) return true;
-        if (!P.same_nl && P.has_A2c && 0.5 * (P.R2c * P.R2c) * (n1 * n2) > 80.0) return true;
+// h1, h2: the norms rounded to FP32. Nearly every pair is settled by them: a difference above 2e-5 of the larger (170
+// times the rounding) and above 2e-4, and arguments below 79.9, leave no doubt, and no FP64 instruction is issued (FP64
+// pipe 48 % busy with these tests in square wells, 67 % in gaussian ones, before). diag: n1 is n2, not far.
+__device__ __forceinline__ bool nl_needs_fp64(const DevParams& P, const DevParamsDS& Q, const double& n1, const double& n2,
+                                              float h1, float h2, bool diag, bool& far) {
+    const float d = fabsf(h1 - h2), np = h1 * h2;
+    bool sure = diag || (d > 2.0e-5f * fmaxf(h1, h2) && d > 2.0e-4f);
+    if (!Q.square) {
+        if (Q.has_A2a) sure = sure && Q.R2a2h.h * np < 79.9f;
+        if (!Q.same_nl && Q.has_A2c) sure = sure && Q.R2c2h.h * np < 79.9f;
     }
-    return false;
+    if (sure) {
+        far = !diag;
+        return false;
+    }
+    const int t = nl_exact_tests(n1, n2, !Q.square && Q.has_A2a ? P.R2a : 0.0, !Q.square && !Q.same_nl && Q.has_A2c ? P.R2c : 0.0);
+    far = t & 1;
+    return t & 2;
 }
 
 // compute_soc_contribution (SpinOrbitFunctional.cpp:111-138) in double-single: sv = (re, im) of
@@ -629,8 +649,10 @@ __device__ __forceinline__ ds4 make_stored<ds4>(ds re, ds im) {
 // (high-symmetry k, where |k + G_i| = |k + G_j| in exact arithmetic and the rounding of the FP64
 // norms takes the reference's far branch, dividing one rounding-level difference by another) is
 // formed by the FP64 element instead: double-single cannot follow that cancellation.
+// CTAs per SM: bound by issue, which the registers of three CTAs kept 56 % busy; 2000 k: Si nonlocal 0.62 -> 0.42 ms,
+// InP 0.52 -> 0.41, Ge (gaussian) 1.64 -> 1.01 with the norms' tests out of the FP64 pipe and these bounds.
 template <typename SO>
-__global__ void __launch_bounds__(256) k_assemble_tiles_ds(const DevParams P, const DevParamsDS Q, const float4* __restrict__ Vloc32,
+__global__ void __launch_bounds__(256, sizeof(SO) == 8 ? 5 : 4) k_assemble_tiles_ds(const DevParams P, const DevParamsDS Q, const float4* __restrict__ Vloc32,
                                                            const float4* __restrict__ phNL32, const float2* __restrict__ rows32,
                                                            const cx<double>* __restrict__ Vloc, const double2* __restrict__ phNL,
                                                            const double* __restrict__ rows,
@@ -661,10 +683,10 @@ __global__ void __launch_bounds__(256) k_assemble_tiles_ds(const DevParams P, co
         te.at(el, il, jl);
         const int i = ti * 32 + il, j = tj * 32 + jl;
         {
-            const double  n1 = si.nk[il], n2 = sj.nk[jl];
+            const double &n1 = si.nk[il], &n2 = sj.nk[jl];
             bool          far;
             SO            v;
-            if (nl_needs_fp64(P, n1, n2, far)) {
+            if (nl_needs_fp64(P, Q, n1, n2, si.ds[RF_NK][il].x, sj.ds[RF_NK][jl].x, i == j, far)) {
                 v = stored(Hb, scalar_element<true>(P, Vloc, phNL, rows, b, i, j));
             } else {
                 const RowDS   Ri{&si.ds[0][il]}, Rj{&sj.ds[0][jl]};
@@ -788,9 +810,9 @@ __global__ void __launch_bounds__(256) k_assemble_soc_tiles(const DevParams P, c
                 if (i == j) hr = ds_add(hr, rd(Ri32, RF_KIN));
                 fp64 = false;
                 if (NL) {
-                    const double n1 = st[0].nk[il], n2 = st[1].nk[jl];
-                    bool         far;
-                    fp64 = nl_needs_fp64(P, n1, n2, far);
+                    const double &n1 = st[0].nk[il], &n2 = st[1].nk[jl];
+                    bool          far;
+                    fp64 = nl_needs_fp64(P, Q, n1, n2, st[0].ds[RF_NK][il].x, st[1].ds[RF_NK][jl].x, i == j, far);
                     if (!fp64) {
                         const float4 pn = phNL32[(size_t)j * N + i];
                         ds           vr, vi;
