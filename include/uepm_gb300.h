@@ -220,7 +220,7 @@ int uepm_measure_peak(int precision, double* tflops);
  *                 autotuner keeps the context's value.
  *   tensor_cores  0 (automatic): the mixed path's complex contractions run on the tensor cores
  *                 (tcgen05) where they apply: the blocked reduction's panel updates (TF32 with
- *                 hi/lo operand splits, FP32-level products) and, from order 150, the Rayleigh-Ritz
+ *                 hi/lo operand splits, FP32-level products) and, with rows and vectors enough, the Rayleigh-Ritz
  *                 product H X (BF16 integer slices of H and X, exact to double-single level);
  *                 1: every product on the FP32 pipe (SIMT). Kept by the autotuner.
  *   streams       0 (automatic): a mixed-precision uepm_solve_device / uepm_solve of 1024 or more

@@ -155,9 +155,17 @@ struct SparseV {
 };
 // half > 0: H is quaternionic, only its first half = n / 2 rows are formed, and the vectors come in pairs
 // (launch_backtransform_quat's); the other rows of Y follow from those.
-// tensor_cores: a complex dense H of order >= kRefineTcMinN takes Y = H X on the tensor cores
-// (refine_tc.cu); status gets UEPM_K_NOCONVERGE there if a bounded wait gives up.
-constexpr int kRefineTcMinN = 150;
+// tensor_cores: a complex dense H takes Y = H X on the tensor cores (refine_tc.cu) where refine_tc_pays; status
+// gets UEPM_K_NOCONVERGE there if a bounded wait gives up.
+//
+// A 128-row tile takes the tensor-core kernel the same time whatever the number of vectors (slicing H binds it): a fixed
+// part and one that grows with the order n. The FP32-pipe form's time goes with the rows nr, the padded vectors mp
+// and n. Projection of 1000 matrices, FP32 pipe against tensor cores, ms: n = 113 mp = 12 0.33 / 0.39, 16 0.41 / 0.41, 20
+// 0.51 / 0.44; 137 20 0.70 / 0.79; 181 12 0.76 / 0.89, 20 1.17 / 0.98; 229 12 1.10 / 1.13, 20 1.79 / 1.24; 338 12 2.24 /
+// 2.11; quaternionic (nr = n / 2) 274 12 0.88 / 1.26, 20 1.40 / 1.40; 362 12 1.54 / 1.61, 16 1.85 / 1.73.
+inline bool refine_tc_pays(int n, int nr, int mp) {
+    return 2ll * nr * mp * n >= 128ll * ((nr + 127) / 128) * (17ll * n + 1200);
+}
 template <typename S>
 void launch_refine_project(const typename Split<S>::type* H, int n, int ld, size_t mstride, const cx<float>* X32, int m,
                            S* work, S* small, int batch, cudaStream_t s, const SparseV& sv, int* status = nullptr,
