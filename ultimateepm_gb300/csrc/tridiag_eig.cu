@@ -697,11 +697,11 @@ template <typename T>
 void launch_invit(const T* d, const T* e, const T* ev, int ev_ld, int n, int nb, T* work, T* z, int* status, int batch,
                   cudaStream_t s, int cap) {
     const size_t smem = invit_smem_bytes<T>(n, std::min(nb, 32));
-    // shared memory where at least four warps fit per SM; beyond that the latency-bound recurrences
-    // run better from the L1/L2-cached workspace at higher occupancy (FP32, 2000 k: Ge SOC n = 362
-    // 1.9 -> 1.6 ms, one warp per SM in shared memory; Si n = 137 0.13 ms in shared memory against
-    // 0.18 from the workspace)
-    if (smem <= 56 * 1024 || (sizeof(T) == 8 && smem <= 200 * 1024)) {
+    // FP32: shared memory where two matrices fit an SM, from the L1/L2-cached workspace beyond (one warp per SM in shared
+    // memory leaves it idle: n = 362, 20 vectors, 2000 matrices 1.9 ms against 1.6). ms in the workspace against
+    // shared memory, 400 and 6000 matrices: n = 178, 20 vectors (3 per SM) 0.24 / 0.13 and 1.21 / 1.06; 229, 20 (2 per SM)
+    // 0.28 / 0.10 and 1.42 / 0.91; 338, 20 0.59 / 0.25 and 3.85 / 2.63.
+    if (smem <= 112 * 1024 || (sizeof(T) == 8 && smem <= 200 * 1024)) {
         auto kern = k_invit<T, true>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<batch, 32, smem, s>>>(d, e, ev, ev_ld, n, nb, work, z, status, batch, cap);
