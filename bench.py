@@ -288,7 +288,7 @@ def run_ours(args):
     # Each figure belongs to the kernel named beside it and holds until that kernel changes: the
     # mixed path's k_tridiag_reg_local (profiles/k_tridiag_si137_2000k.md) and the FP64 path's
     # k_tridiag<double> (profiles/launches_si137_2000k.md); re-capture them whenever either is edited.
-    traffic = {"tridiag_fp32": 83.66e6, "tridiag_fp64": 9.108e9}
+    traffic = {"tridiag_fp32": 81.99e6, "tridiag_fp64": 7.286e9}
     traffic_kernel = {"tridiag_fp32": "k_tridiag_reg_local (register-resident FP32 reduction, n = 137)",
                       "tridiag_fp64": "k_tridiag<double> (persistent global-memory FP64 reduction, n = 137)"}
     peak64 = C.c_double()
@@ -635,9 +635,9 @@ def run_configs(seed: int = 20261203):
         tc_block = None
         if soc:
             # the mixed solve's kernels on 2000 of the k-points, CUDA events per kernel (a separate,
-            # profiled solve: the timed one above runs without events), with the tensor-core kernels'
-            # work: the reduction's panel updates (tcgen05 kind::tf32) and Y = H X (kind::f16 on BF16
-            # slices: 36 slice pairs x 2 x 128 x N x K per 128-row tile)
+            # profiled solve: the timed one above runs without events), with the tensor-core kernel's
+            # work: Y = H X (kind::f16 on BF16 slices: 36 slice pairs x 2 x 128 x N x K per 128-row tile of
+            # the rows that the quaternion form computes, the first n / 2)
             ctx = api._Context(m, G, nl, soc, N.UEPM_PREC_MIXED)
             # one stream, so that each kernel's events time that kernel alone (the timed solve above
             # runs its chunks on two streams)
@@ -658,12 +658,11 @@ def run_configs(seed: int = 20261203):
             mpad = (mm + 3) // 4 * 4
             ncol = (2 * mpad + 15) // 16 * 16
             kdim = 32 * ((n + 15) // 16)
-            bf16_flop = 36 * 2 * 128 * ncol * kdim * ((n + 127) // 128) * 2000
+            bf16_flop = 36 * 2 * 128 * ncol * kdim * ((n // 2 + 127) // 128) * 2000
             rp_ms = prof.get("refine_project", float("nan"))
             tc_block = {
                 "kernels_ms_per_2000_k": {q: round(v, 3) for q, v in prof.items()},
-                "tensor_core_kernels": ["k_tridiag_blocked (panel updates, tcgen05.mma kind::tf32, hi/lo splits)",
-                                        "k_refine_y_tc (Y = H X, tcgen05.mma kind::f16 on exact BF16 slices)"],
+                "tensor_core_kernels": ["k_refine_y_tc (Y = H X, tcgen05.mma kind::f16 on exact BF16 slices)"],
                 "refine_project_bf16_issued_tflops": bf16_flop / (rp_ms * 1e-3) / 1e12,
                 "refine_project_note": "refine_project = k_refine_y_tc + the double-single S, A kernel; BF16 "
                                        "flops issued by the slice products over that time",
