@@ -189,7 +189,7 @@ __device__ __forceinline__ void product(const S* A, int ld, int m, const S* v, i
 // SMs idle. The product's NW virtual warps and the update's elements are dealt out over the cluster, the
 // partial products and the next column go to every CTA's shared memory (distributed shared memory), and the
 // rest is done by every CTA for itself; rank 0 writes the outputs. Every sum keeps its order, so the results
-// are the same bits for every CL. Two cluster barriers per column.
+// are the same bits for every CL. Two cluster barriers per column, and one before the first.
 template <typename S, int NT, int MAXT, bool SMEM, int CL = 1>
 __global__ void __launch_bounds__(NT, SMEM || CL > 1 ? 1 : tridiag_min_blocks<S, MAXT>()) k_tridiag(S* __restrict__ H, int n, int ldg, size_t mstride,
                                                 typename ST<S>::R* __restrict__ dOut, typename ST<S>::R* __restrict__ eOut,
@@ -245,6 +245,9 @@ __global__ void __launch_bounds__(NT, SMEM || CL > 1 ? 1 : tridiag_min_blocks<S,
         xc[k]       = r < n ? ldc(A + r) : ST<S>::zero();
         if (r >= 2 && r < n) ss += ST<S>::norm(xc[k]);
     }
+    // Every CTA of the cluster has read column 0 before rank 0 writes its reflector there, and has started before
+    // a peer's to_all writes into its shared memory.
+    if constexpr (CL > 1) sync_cluster();
     for (int i = 0; i < n - 1; ++i) {
         const int o = i + 1, m = n - o;
         S*        col = A + (size_t)i * ld + o;
