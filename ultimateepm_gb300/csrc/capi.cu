@@ -256,9 +256,10 @@ int check_launch() {
 
 
 // One chunk of c k-points through the pipeline, FP64 (S = double for real H, cx<double> otherwise)
-// or mixed precision (FP32 reduction in Lower<S>, FP64 Rayleigh-Ritz in S).
+// or mixed precision (FP32 reduction in Lower<S>, FP64 Rayleigh-Ritz in S). An error where a kernel without a
+// substitute cannot run: what follows it would work on whatever the workspace holds.
 template <typename S>
-void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const double* kk, int c, int nb, int m, bool vec,
+int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const double* kk, int c, int nb, int m, bool vec,
                double* E, cx<double>* Xo, double* gr, int* st, cudaStream_t s) {
     using S32            = typename Lower<S>::type;
     const int    n       = f.n;
@@ -306,7 +307,7 @@ void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const do
                 launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, P, kk, ctx->d_G, gr, c, s);
             }
         }
-        return;
+        return UEPM_OK;
     }
     if (ctx->precision != UEPM_PREC_MIXED) {
         {
@@ -335,7 +336,7 @@ void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const do
             ProfScope p(ctx, s, KK_BACKTRANSFORM);
             launch_backtransform<S>(H, n, n, mstride, tq, z, nb, Xo, P, kk, ctx->d_G, gr, c, s, ctx->tune.vector_lanes);
         }
-        return;
+        return UEPM_OK;
     }
     using SP  = typename Split<S>::type;
     auto* H32 = reinterpret_cast<S32*>(ws + L.H32);
@@ -379,7 +380,10 @@ void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const do
         const size_t qs = (size_t)N * N;
         {
             ProfScope p(ctx, s, KK_TRIDIAG32);
-            launch_tridiag_tri<qt<float>>(HQ, N, N, qs, d, e, qq, st, c, s);
+            if (!launch_tridiag_tri<qt<float>>(HQ, N, N, qs, d, e, qq, st, c, s)) {
+                set_error("the quaternion reduction of order " + std::to_string(N) + " could not be launched");
+                return UEPM_ERR_CUDA;
+            }
         }
         {
             ProfScope p(ctx, s, KK_BISECT);
@@ -435,6 +439,7 @@ void run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const do
         ProfScope p(ctx, s, KK_REFINE_VECTORS);
         launch_refine_vectors<S>(n, m, nb, X32, W, Xo, gr, P, kk, ctx->d_G, c, s);
     }
+    return UEPM_OK;
 }
 
 }  // namespace
@@ -553,8 +558,9 @@ int enqueue_solve(uepm_ctx* ctx, const SolvePlan& sp, const double* d_k, size_t 
             gr = want_grad ? reinterpret_cast<double*>(wsq + L.fg) : nullptr;
         }
         const int nf = form_bands(f, nb);
-        if (f.real) run_chunk<double>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
-        else run_chunk<cx<double>>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
+        rc = f.real ? run_chunk<double>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq)
+                    : run_chunk<cx<double>>(ctx, f, L, wsq, kk, c, nf, sp.m, want_vec || want_grad, E, Xo, gr, st, sq);
+        if (rc) break;
         if (f.scalar)
             launch_spin_pairs(E, Xo, gr, ctx->N, nf, nb, c, d_E + off * nb,
                               want_vec ? reinterpret_cast<cx<double>*>(d_X) + off * nb * n : nullptr,

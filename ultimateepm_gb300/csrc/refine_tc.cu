@@ -335,7 +335,8 @@ bool launch_refine_y_tc(const ds4* H, int n, int ld, size_t mstride, const cx<fl
     const int N = (2 * mp + 15) / 16 * 16;
     if (n < 2 || n > 1024 || m > mp || N > kYtNmax || mp > kYtNmax / 2) return false;
     auto kern = k_refine_y_tc;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYtSmem) != cudaSuccess) return false;
+    const Refusal refuse;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYtSmem) != cudaSuccess) return refuse();
     const int nr    = half ? half : n;
     const int ntile = (nr + kYtM - 1) / kYtM;
     kern<<<batch * ntile, kYtNT, kYtSmem, s>>>(H, n, ld, mstride, X32, m, mp, N, reinterpret_cast<float4*>(work), ystride,

@@ -685,7 +685,8 @@ bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>:
     const size_t smem = nc ? BlkSmem<S>::bytes_tc(n, nc) : BlkSmem<S>::bytes(n);
     if (smem > 227 * 1024) return false;
     auto kern = k_tridiag_blocked<S>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+    const Refusal refuse;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -215,11 +215,9 @@ bool launch_tridiag_cluster(S* H, int n, int ld, size_t mstride, typename ST<S>:
     if (!C || batch <= 0) return false;
     const size_t smem = cluster_smem<S>(n, C);
     auto         kern = k_tridiag_cluster<S>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
-    if (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    const Refusal refuse;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
+    if (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return refuse();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id               = cudaLaunchAttributeClusterDimension;
@@ -233,13 +231,10 @@ bool launch_tridiag_cluster(S* H, int n, int ld, size_t mstride, typename ST<S>:
     cfg.numAttrs           = 1;
     int maxc               = 0;
     cfg.gridDim            = dim3(C * std::min(batch, 1024));
-    if (cudaOccupancyMaxActiveClusters(&maxc, kern, &cfg) != cudaSuccess || maxc <= 0) {
-        cudaGetLastError();
-        return false;
-    }
+    if (cudaOccupancyMaxActiveClusters(&maxc, kern, &cfg) != cudaSuccess || maxc <= 0) return refuse();
     cfg.gridDim = dim3(C * std::min(batch, maxc));
     const int ncol = (n + C - 1) / C;
-    if (cudaLaunchKernelEx(&cfg, kern, H, n, ld, mstride, d, e, tq, status, batch, ncol) != cudaSuccess) return false;
+    if (cudaLaunchKernelEx(&cfg, kern, H, n, ld, mstride, d, e, tq, status, batch, ncol) != cudaSuccess) return refuse();
     count_launch();
     return true;
 }

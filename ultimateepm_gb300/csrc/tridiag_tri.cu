@@ -437,11 +437,12 @@ bool tri_launch(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, 
     while (nres > 2 && TriLayout<S>(n, nres, NT).total > kTriSmem - 1024) --nres;
     const size_t smem = TriLayout<S>(n, nres, NT).total;
     auto         kern = nres == n ? k_tridiag_tri<S, NT, MINB, false> : k_tridiag_tri<S, NT, MINB, true>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+    const Refusal refuse;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, NT, smem) != cudaSuccess || fit < 1) return false;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, NT, smem) != cudaSuccess || fit < 1) return refuse();
     const int grid = std::min(batch, std::max(1, sms) * fit);
     kern<<<grid, NT, smem, s>>>(H, n, nres, ld, mstride, d, e, tq, status, batch);
     count_launch();

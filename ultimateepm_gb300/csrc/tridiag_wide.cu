@@ -14,9 +14,10 @@ template <typename S, int MAXT, int CL>
 bool wide_launch(S* H, int n, int ld, size_t mstride, double* d, double* e, S* tq, int* status, int batch, cudaStream_t s) {
     constexpr int NT   = 256;
     const size_t  smem = sizeof(S) * (size_t)(3 + NT / 32) * n;
+    const Refusal refuse;
     auto          kern = k_tridiag<S, NT, MAXT, false, CL>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return false;
+        return refuse();
     cudaLaunchConfig_t  cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id               = cudaLaunchAttributeClusterDimension;
@@ -29,7 +30,7 @@ bool wide_launch(S* H, int n, int ld, size_t mstride, double* d, double* e, S* t
     cfg.stream             = s;
     cfg.attrs              = at;
     cfg.numAttrs           = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, H, n, ld, mstride, d, e, tq, status, batch) != cudaSuccess) return false;
+    if (cudaLaunchKernelEx(&cfg, kern, H, n, ld, mstride, d, e, tq, status, batch) != cudaSuccess) return refuse();
     count_launch();
     return true;
 }

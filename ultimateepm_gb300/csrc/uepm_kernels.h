@@ -9,6 +9,16 @@
 
 namespace uepm {
 
+// For a launcher that returns false with nothing launched: takes back the error of the call that failed, so that
+// the caller's other kernel does not answer for it. An error that was pending before is left for the caller.
+struct Refusal {
+    bool clean = cudaPeekAtLastError() == cudaSuccess;
+    bool operator()() const {
+        if (clean) cudaGetLastError();
+        return false;
+    }
+};
+
 void count_launch(int n = 1);
 
 // assemble.cu: H(k) in FULL column-major storage (both triangles). SO = double (real H) or
