@@ -253,7 +253,10 @@ int check_launch() {
     }
     return UEPM_OK;
 }
-
+int not_launched(const char* what, int n) {
+    set_error(std::string("the ") + what + " of order " + std::to_string(n) + " could not be launched");
+    return UEPM_ERR_CUDA;
+}
 
 // One chunk of c k-points through the pipeline, FP64 (S = double for real H, cx<double> otherwise)
 // or mixed precision (FP32 reduction in Lower<S>, FP64 Rayleigh-Ritz in S). An error where a kernel without a
@@ -293,7 +296,7 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
             }
             {
                 ProfScope p(ctx, s, KK_BISECT);
-                launch_bisect<double>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st);
+                if (!launch_bisect<double>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st)) return not_launched("bisection", N);
                 launch_pair_values(ev, nz, E, nb, c, s);
             }
             if (vec) {
@@ -324,7 +327,7 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
         }
         {
             ProfScope p(ctx, s, KK_BISECT);
-            launch_bisect<double>(d, e, n, nb, E, nb, c, s, ctx->tune.max_iter, st);
+            if (!launch_bisect<double>(d, e, n, nb, E, nb, c, s, ctx->tune.max_iter, st)) return not_launched("bisection", n);
         }
         if (vec) {
             auto* work = reinterpret_cast<double*>(ws + L.work);
@@ -380,14 +383,11 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
         const size_t qs = (size_t)N * N;
         {
             ProfScope p(ctx, s, KK_TRIDIAG32);
-            if (!launch_tridiag_tri<qt<float>>(HQ, N, N, qs, d, e, qq, st, c, s)) {
-                set_error("the quaternion reduction of order " + std::to_string(N) + " could not be launched");
-                return UEPM_ERR_CUDA;
-            }
+            if (!launch_tridiag_tri<qt<float>>(HQ, N, N, qs, d, e, qq, st, c, s)) return not_launched("quaternion reduction", N);
         }
         {
             ProfScope p(ctx, s, KK_BISECT);
-            launch_bisect<float>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st);
+            if (!launch_bisect<float>(d, e, N, nz, ev, nz, c, s, ctx->tune.max_iter, st)) return not_launched("bisection", N);
         }
         {
             ProfScope p(ctx, s, KK_INVIT);
@@ -411,7 +411,7 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
     }
     {
         ProfScope p(ctx, s, KK_BISECT);
-        launch_bisect<float>(d, e, n, m, ev, m, c, s, ctx->tune.max_iter, st);
+        if (!launch_bisect<float>(d, e, n, m, ev, m, c, s, ctx->tune.max_iter, st)) return not_launched("bisection", n);
     }
     {
         ProfScope p(ctx, s, KK_INVIT);

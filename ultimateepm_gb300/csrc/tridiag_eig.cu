@@ -361,24 +361,29 @@ static bool bisect_launch(const T* d, const T* e, int n, int nb, T* ev, int ev_l
 // 882 -> 266 (16), 3200 883 -> 464 and 8000 883 -> 661 (4), 16000 883 -> 797 (4, then 1 in the FP64 phase),
 // n = 113 24000 1046 -> 760, n = 181 1800 1159 -> 430 (8); FP32 n = 137, 960 98 -> 29 (32), 4800 98 -> 45 (8),
 // 16000 105 -> 86 (4). Beyond the last threshold one lane is fastest (65536 FP64 values: 2091 against 2152).
+//
+// A CTA stages every matrix that its values touch: one lane per value and few bands per matrix need more shared memory
+// than it takes. The next form with more lanes then stands in, which holds fewer matrices: 42000 to 80000 FP64 values
+// in ms, the 4-lane form against 32 lanes (which takes 31 / 5 of the Sturm counts): n = 137 with 2 and 4 bands 2.7 / 9.1 and
+// 2.5 / 14.3, 181 with 4 2.6 / 10.2, 113 with 4 1.4 / 6.8; with one band, where 4 lanes do not fit either, 8 lanes 3.9 / 8.5.
+// 32 lanes fit every order up to 512.
 template <typename T>
-void launch_bisect(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap, int* status) {
-    if (batch <= 0) return;
+bool launch_bisect(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap, int* status) {
+    if (batch <= 0) return true;
     const long long items = (long long)batch * nb;
 #define UEPM_BIS(P_, Q_) bisect_launch<T, P_, Q_>(d, e, n, nb, ev, ev_ld, batch, s, cap, status)
     if constexpr (sizeof(T) == 8) {
-        if (items > 512 && items <= 1024 && UEPM_BIS(16, 16)) return;
-        if (items > 1024 && items <= 2400 && UEPM_BIS(8, 8)) return;
-        if (items > 2400 && items <= 12000 && UEPM_BIS(4, 4)) return;
-        if (items > 12000 && items <= 40000 && UEPM_BIS(4, 1)) return;
-        if (items > 40000 && UEPM_BIS(1, 1)) return;
+        if (items > 40000 && UEPM_BIS(1, 1)) return true;
+        if (items > 12000 && UEPM_BIS(4, 1)) return true;
+        if (items > 2400 && UEPM_BIS(4, 4)) return true;
+        if (items > 1024 && UEPM_BIS(8, 8)) return true;
+        if (items > 512 && UEPM_BIS(16, 16)) return true;
     } else {
-        if (items > 1024 && items <= 6000 && UEPM_BIS(8, 8)) return;
-        if (items > 6000 && items <= 24000 && UEPM_BIS(4, 4)) return;
-        if (items > 24000 && UEPM_BIS(1, 1)) return;
+        if (items > 24000 && UEPM_BIS(1, 1)) return true;
+        if (items > 6000 && UEPM_BIS(4, 4)) return true;
+        if (items > 1024 && UEPM_BIS(8, 8)) return true;
     }
-    // few values, or orders whose staging leaves room for few matrices per CTA
-    UEPM_BIS(32, 32);
+    return UEPM_BIS(32, 32);
 #undef UEPM_BIS
 }
 
@@ -712,8 +717,8 @@ void launch_invit(const T* d, const T* e, const T* ev, int ev_ld, int n, int nb,
     count_launch();
 }
 
-template void launch_bisect<double>(const double*, const double*, int, int, double*, int, int, cudaStream_t, int, int*);
-template void launch_bisect<float>(const float*, const float*, int, int, float*, int, int, cudaStream_t, int, int*);
+template bool launch_bisect<double>(const double*, const double*, int, int, double*, int, int, cudaStream_t, int, int*);
+template bool launch_bisect<float>(const float*, const float*, int, int, float*, int, int, cudaStream_t, int, int*);
 template void launch_invit<double>(const double*, const double*, const double*, int, int, int, double*, double*, int*, int,
                                    cudaStream_t, int);
 template void launch_invit<float>(const float*, const float*, const float*, int, int, int, float*, float*, int*, int,

@@ -104,9 +104,9 @@ void launch_tridiag_reg(cx<float>* H, int n, int ld, size_t mstride, float* d, f
 void launch_tridiag_reg_local(const float* V32, const cx<double>* Vloc, const double* rows, float* H, int n, int ld,
                               size_t mstride, float* d, float* e, float* tq, int* status, int batch, cudaStream_t s);
 
-// tridiag_eig.cu
+// tridiag_eig.cu (false, with nothing launched, for orders beyond 512)
 template <typename T>
-void launch_bisect(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap = 0,
+bool launch_bisect(const T* d, const T* e, int n, int nb, T* ev, int ev_ld, int batch, cudaStream_t s, int cap = 0,
                    int* status = nullptr);
 template <typename T>
 void launch_invit(const T* d, const T* e, const T* ev, int ev_ld, int n, int nb, T* work, T* z, int* status, int batch,
