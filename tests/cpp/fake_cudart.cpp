@@ -1,8 +1,10 @@
 // fake_cudart.cpp -- stands in for the CUDA runtime by LD_PRELOAD (tests/fake_runtime.py), so that the host side of
 // a solve runs without a GPU: device memory is the host's, kernels do nothing, and every launch and every limit on
-// a kernel's dynamic shared memory is written down. A call can be made to fail (fake_refuse).
+// a kernel's dynamic shared memory is written down. A launch above its kernel's limit fails, as does a limit above
+// the device's, and other calls can be made to fail (fake_refuse).
 #include <cuda_runtime_api.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -14,7 +16,9 @@ struct Call {
     size_t smem;
     void*  stream;
 };
+constexpr size_t kSmemDefault = 48 * 1024, kSmemOptin = 227 * 1024;
 std::map<const void*, std::string> g_names;  // host stub -> kernel
+std::map<const void*, size_t>      g_limits;
 std::string g_log, g_refuse;
 cudaError_t g_last = cudaSuccess;
 Call        g_call;
@@ -28,7 +32,7 @@ bool refused(const char* call, const void* f) {
 }
 cudaError_t fail(cudaError_t e) { return g_last = e; }
 cudaError_t launched(const void* f, dim3 g, dim3 b, size_t smem) {
-    if (refused("launch", f)) return fail(cudaErrorInvalidValue);
+    if (refused("launch", f) || smem > std::max(kSmemDefault, g_limits[f])) return fail(cudaErrorInvalidValue);
     g_log += "launch " + name_of(f) + " " + std::to_string(g.x) + " " + std::to_string(b.x * b.y) + " " + std::to_string(smem) + "\n";
     return cudaSuccess;
 }
@@ -65,7 +69,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     if (refused("cudaFuncSetAttribute", f)) return fail(cudaErrorInvalidValue);
-    if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) g_log += "smem " + name_of(f) + " " + std::to_string(v) + "\n";
+    if (a != cudaFuncAttributeMaxDynamicSharedMemorySize) return cudaSuccess;
+    if ((size_t)v > kSmemOptin) return fail(cudaErrorInvalidValue);
+    g_limits[f] = v;
+    g_log += "smem " + name_of(f) + " " + std::to_string(v) + "\n";
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int, size_t, unsigned) {

@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(kProjNT, proj_min_blocks<S, SPARSE, YDONE>()) 
 // The Jacobi sweeps rotate m/2 disjoint pairs at once (round-robin tournament order), the lanes of
 // the warp computing the pairs' rotations and then sharing the row/column updates, so FP64
 // instructions are issued with most lanes busy.
+// Two warps per CTA, one where the shared memory does not hold two matrices (complex order 40: 119 KB each).
 constexpr int kSmallWarps = 2;
 
 // shared memory of one warp's matrix: L, C, V (m x (m+1) scalars each), 4 rotation arrays, the
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small_eigh(S* __restrict__
                                                                  int want_w, int* __restrict__ status, int batch, int cap) {
     using R         = double;
     const int warp  = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b     = blockIdx.x * kSmallWarps + warp;
+    const int b     = blockIdx.x * (blockDim.x >> 5) + warp;
     const int mp    = m + 1;                       // padded row length
     const int me    = (m + 1) & ~1;                // m rounded up to even (tournament size)
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -772,11 +773,11 @@ void launch_refine_project(const typename Split<S>::type* H, int n, int ld, size
 
 template <typename S>
 void launch_small_eigh(S* small, int m, int nb, double* Eout, S* W, int* status, int batch, cudaStream_t s, int cap) {
-    const size_t smem = small_eigh_warp_bytes<S>(m) * kSmallWarps;
-    auto         kern = k_small_eigh<S>;
+    const int    warps = small_eigh_warp_bytes<S>(m) * kSmallWarps <= kMaxDynamicSmem ? kSmallWarps : 1;
+    const size_t smem  = small_eigh_warp_bytes<S>(m) * warps;
+    auto         kern  = k_small_eigh<S>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<(batch + kSmallWarps - 1) / kSmallWarps, 32 * kSmallWarps, smem, s>>>(small, m, nb, Eout, W != nullptr, status,
-                                                                              batch, cap);
+    kern<<<(batch + warps - 1) / warps, 32 * warps, smem, s>>>(small, m, nb, Eout, W != nullptr, status, batch, cap);
     count_launch();
 }
 

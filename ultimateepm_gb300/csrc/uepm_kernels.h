@@ -19,6 +19,10 @@ struct Refusal {
     }
 };
 
+// The dynamic shared memory that a CTA may take: 227 KB, less what the kernels hold as static shared memory (800 bytes
+// at most).
+constexpr size_t kMaxDynamicSmem = 226 * 1024;
+
 void count_launch(int n = 1);
 
 // assemble.cu: H(k) in FULL column-major storage (both triangles). SO = double (real H) or
