@@ -10,7 +10,8 @@ SRC = os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")
 
 
 def run(tmp_path, *cases):
-    """A case: material, shells, bands, k, and optionally nl, soc, mixed, tuning, autotune, refuse. Returns for each its error
+    """A case: material, shells, bands, k, and optionally plane_waves (the first so many of the basis), nl, soc, mixed,
+    vectors, tuning, autotune, refuse. Returns for each its error
     (None: it was solved), its launches (kernel, grid, threads, shared memory) and the shared-memory limits set."""
     from ultimateepm_gb300 import build
 
@@ -39,7 +40,7 @@ def _solve(c, fake):
 
     ms = api.Materials()
     ms.load_material_parameters(os.path.join(ROOT, "params", "materials.yaml"))
-    ctx = api._Context(ms.materials[c["material"]], api.generate_basis_vectors(c["shells"]), c.get("nl", False), c.get("soc", False),
+    ctx = api._Context(ms.materials[c["material"]], api.generate_basis_vectors(c["shells"])[:c.get("plane_waves")], c.get("nl", False), c.get("soc", False),
                        N.UEPM_PREC_MIXED if c.get("mixed") else N.UEPM_PREC_FP64)
     N.check(N.load().uepm_ctx_set_tuning(ctx.h, C.byref(N.UepmTuning(**c.get("tuning", {})))))
     if "autotune" in c:

@@ -3,7 +3,7 @@ and the other kernel runs; where there is no other kernel the solve fails, inste
 workspace holds."""
 import fake_runtime
 
-GE = dict(material="Ge", shells=6, bands=8, nl=True, soc=True)
+GE = dict(material="Ge", shells=10, bands=8, nl=True, soc=True)
 
 
 def test_the_fake_runtime_sees_an_ordinary_solve(native, tmp_path):

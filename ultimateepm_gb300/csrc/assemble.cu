@@ -921,7 +921,7 @@ void launch_assemble(const DevParams& P, const cx<double>* Vloc, const double2* 
     dim3         grd(T * (T + 1) / 2, batch);
     const size_t smem = sizeof(SO) * 4 * 32 * 33;
     auto         kern = P.nl ? k_assemble_soc_tiles<true, false, false, SO> : k_assemble_soc_tiles<false, false, false, SO>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, H, ld, mstride, H32, mstride32, batch, DevParamsDS{}, nullptr,
                                 nullptr, nullptr, nullptr, nullptr, 0);
     count_launch();
@@ -951,7 +951,7 @@ void launch_assemble_soc_ds(const DevParams& P, const DevParamsDS& Q, const floa
     const size_t smem = sizeof(SO) * (HQ ? 2 : 4) * 32 * 33 + 2 * sizeof(StagedRows);
     auto         kern = HQ ? (P.nl ? k_assemble_soc_tiles<true, true, true, SO> : k_assemble_soc_tiles<false, true, true, SO>)
                            : (P.nl ? k_assemble_soc_tiles<true, true, false, SO> : k_assemble_soc_tiles<false, true, false, SO>);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, H, ld, mstride, H32, mstride32, batch, Q, Vloc32, phNL32, phSO32,
                                 rows32, HQ, mstrideq);
     count_launch();
@@ -963,7 +963,7 @@ void launch_assemble_quat(const DevParams& P, const cx<double>* Vloc, const doub
     dim3         grd(T * (T + 1) / 2, batch), blk(32, 8);
     const size_t smem = sizeof(SO) * 2 * 32 * 33;
     auto         kern = P.nl ? k_assemble_soc_tiles<true, false, true, SO> : k_assemble_soc_tiles<false, false, true, SO>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<grd, blk, smem, s>>>(P, Vloc, phNL, phSO, rows, nullptr, 0, 0, nullptr, 0, batch, DevParamsDS{}, nullptr, nullptr,
                                 nullptr, nullptr, HQ, mstrideq);
     count_launch();

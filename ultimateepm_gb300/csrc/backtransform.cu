@@ -221,7 +221,7 @@ static void bt_launch(const S* H, int n, int ld, size_t mstride, const S* tq, co
     const int     cap   = std::max(ldv, std::min(total, (int)(kBtStageBytes / sizeof(S))));
     const size_t  smem  = sizeof(S) * ((size_t)cap + n);
     auto          kern  = k_backtransform<S, LPV, T>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<batch, 32 * warps, smem, s>>>(H, n, ld, mstride, tq, z, nb, cap, Xout, P, d_k, d_G, grad, batch, nbo);
     count_launch();
 }

@@ -141,7 +141,7 @@ extern "C" int uepm_dielectric_sums_device(const double* d_Xk, const double* d_X
         set_error(std::string("uepm_dielectric_sums_device: ") + cudaGetErrorString(e));
         return UEPM_ERR_NOMEM;
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_dielectric_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_dielectric_sums, smem);
     k_dielectric_sums<<<grid, kDfThreads, smem, s>>>(reinterpret_cast<const double2*>(d_Xk), reinterpret_cast<const double2*>(d_Xkq),
                                                       d_Ek, d_Ekq, nk, nb, n, first_cond, d_energies, ne, eta, d_weights, part);
     k_dielectric_reduce<<<(ne + 127) / 128, 128, 0, s>>>(part, grid, ne, d_sums);

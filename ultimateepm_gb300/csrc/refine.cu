@@ -740,7 +740,7 @@ static void refine_project_t(const typename Split<S>::type* H, int n, int ld, si
     const int nt = rounds ? (items + 32 * rounds - 1) / (32 * rounds) * 32 : kProjNT;
     if (stage <= kProjStageBytes) {
         auto kern = k_refine_project<S, true, SPARSE, YDONE>;
-        if (stage > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage);
+        allow_smem(kern, stage);
         kern<<<batch, nt, stage, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
     } else {
         k_refine_project<S, false, SPARSE, YDONE><<<batch, nt, 0, s>>>(H, n, ld, mstride, X32, m, work, small, batch, sv, nr);
@@ -776,7 +776,7 @@ void launch_small_eigh(S* small, int m, int nb, double* Eout, S* W, int* status,
     const int    warps = small_eigh_warp_bytes<S>(m) * kSmallWarps <= kMaxDynamicSmem ? kSmallWarps : 1;
     const size_t smem  = small_eigh_warp_bytes<S>(m) * warps;
     auto         kern  = k_small_eigh<S>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<(batch + warps - 1) / warps, 32 * warps, smem, s>>>(small, m, nb, Eout, W != nullptr, status, batch, cap);
     count_launch();
 }

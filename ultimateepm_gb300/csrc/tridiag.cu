@@ -478,7 +478,7 @@ static void tridiag_launch_t(S* H, int n, int ld, size_t mstride, typename ST<S>
     using R           = typename ST<S>::R;
     const size_t smem = sizeof(S) * ((SMEM ? (size_t)n * (n | 1) : 0) + (size_t)(2 + NT / 32) * n);
     auto         kern = k_tridiag<S, NT, MAXT, SMEM>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     int grid = batch;
     if (!SMEM) {
         // automatic: keep the matrices in flight within ~120 MB so that they stay in the 129 MB L2
@@ -505,7 +505,7 @@ static void fused_launch_t(S* H, int n, int ld, size_t mstride, typename ST<S>::
     const size_t  smem = DEFER ? sizeof(S) * (size_t)(5 + NT / 32) * n + sizeof(R) * 7 * (NT / 32)
                                : sizeof(S) * (size_t)(3 + NT / 32) * n + sizeof(R) * 3 * (NT / 32);
     auto          kern = DEFER ? k_tridiag_fused_deferred<S, NT, MAXT> : k_tridiag_fused<S, NT, MAXT>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     // matrices in flight as for the unfused kernel (L2 budget, at least 4 per SM), capped at the
     // kernel's occupancy
     const size_t bytes  = sizeof(S) * (size_t)n * n;

@@ -686,7 +686,7 @@ bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>:
     if (smem > 227 * 1024) return false;
     auto kern = k_tridiag_blocked<S>;
     const Refusal refuse;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
+    if (allow_smem(kern, smem) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -216,7 +216,7 @@ bool launch_tridiag_cluster(S* H, int n, int ld, size_t mstride, typename ST<S>:
     const size_t smem = cluster_smem<S>(n, C);
     auto         kern = k_tridiag_cluster<S>;
     const Refusal refuse;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
+    if (allow_smem(kern, smem) != cudaSuccess) return refuse();
     if (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return refuse();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];

@@ -348,7 +348,7 @@ static bool bisect_launch(const T* d, const T* e, int n, int nb, T* ev, int ev_l
     const size_t smem = (bisect_matrix_bytes<T>(n) + sizeof(BisectMatrix)) * nm;
     if (smem > 96 * 1024) return false;
     auto kern = k_bisect<T, P, Q>;
-    if (smem > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     kern<<<(unsigned)((items + IPB - 1) / IPB), 32 * kBisectWarpsPerBlock, smem, s>>>(d, e, n, nb, ev, ev_ld, batch, cap,
                                                                                    status);
     count_launch();
@@ -708,7 +708,7 @@ void launch_invit(const T* d, const T* e, const T* ev, int ev_ld, int n, int nb,
     // 0.28 / 0.10 and 1.42 / 0.91; 338, 20 0.59 / 0.25 and 3.85 / 2.63.
     if (smem <= 112 * 1024 || (sizeof(T) == 8 && smem <= 200 * 1024)) {
         auto kern = k_invit<T, true>;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern, smem);
         kern<<<batch, 32, smem, s>>>(d, e, ev, ev_ld, n, nb, work, z, status, batch, cap);
     } else {
         const int blocks = (batch + kInvitWarpsPerBlock - 1) / kInvitWarpsPerBlock;

@@ -438,7 +438,7 @@ bool tri_launch(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, 
     const size_t smem = TriLayout<S>(n, nres, NT).total;
     auto         kern = nres == n ? k_tridiag_tri<S, NT, MINB, false> : k_tridiag_tri<S, NT, MINB, true>;
     const Refusal refuse;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return refuse();
+    if (allow_smem(kern, smem) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -16,8 +16,7 @@ bool wide_launch(S* H, int n, int ld, size_t mstride, double* d, double* e, S* t
     const size_t  smem = sizeof(S) * (size_t)(3 + NT / 32) * n;
     const Refusal refuse;
     auto          kern = k_tridiag<S, NT, MAXT, false, CL>;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return refuse();
+    if (allow_smem(kern, smem) != cudaSuccess) return refuse();
     cudaLaunchConfig_t  cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id               = cudaLaunchAttributeClusterDimension;

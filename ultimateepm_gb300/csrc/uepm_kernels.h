@@ -22,6 +22,13 @@ struct Refusal {
 // The dynamic shared memory that a CTA may take: 227 KB, less what the kernels hold as static shared memory (800 bytes
 // at most).
 constexpr size_t kMaxDynamicSmem = 226 * 1024;
+// Lets a kernel be launched with smem bytes of dynamic shared memory. Without asking it gets 48 KB together with its
+// static shared memory.
+template <typename K>
+cudaError_t allow_smem(K kern, size_t smem) {
+    if (smem <= 47 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
 
 void count_launch(int n = 1);
 
