@@ -16,8 +16,8 @@ struct Call {
     size_t smem;
     void*  stream;
 };
-// less 800 bytes, the most that one of the kernels holds as static shared memory
-constexpr size_t kSmemDefault = 48 * 1024 - 800, kSmemOptin = 227 * 1024 - 800;
+// less static shared memory: the most that one of the kernels holds, and that of the kernel with the highest limit
+constexpr size_t kSmemDefault = 48 * 1024 - 800, kSmemOptin = 227 * 1024 - 48;
 std::map<const void*, std::string> g_names;  // host stub -> kernel
 std::map<const void*, size_t>      g_limits;
 std::string g_log, g_refuse;

@@ -29,3 +29,16 @@ def test_fp64_solves_at_the_line(gpu, oracle, mats, key, soc, n):
     ctx.close()
     ref = oracle.band_structure(mats[key], G, ks, 8, nl=False, soc=soc)["E"]
     assert not st.any() and np.abs(E - np.tile(ref, (39, 1))).max() <= 1e-10
+
+
+def test_a_kernel_has_one_limit(native, tmp_path):
+    """The limit is the process's: at every order the same, so that a thread that solves a small order between another
+    thread's limit and its launch does not take shared memory from it."""
+    every = [dict(material=key, shells=s, bands=nb, k=k, nl=nl, soc=soc, mixed=mixed, vectors=True, tuning=dict(reduction=red))
+             for key, nl, soc in (("Ge", True, True), ("GaAs", True, True), ("InP", True, False), ("Ge", True, False)) for s in (6, 10, 13)
+             for nb, k in ((4, 2), (28, 100)) for mixed in (False, True) for red in ((0, 3, 6) if mixed else (0, 2))]
+    limits = {}
+    for _, launches, smem in fake_runtime.run(tmp_path, *every):
+        for kernel, most in smem:
+            limits.setdefault(kernel, set()).add(most)
+    assert len(limits) > 10 and {k: v for k, v in limits.items() if len(v) > 1} == {}

@@ -336,7 +336,7 @@ bool launch_refine_y_tc(const ds4* H, int n, int ld, size_t mstride, const cx<fl
     if (n < 2 || n > 1024 || m > mp || N > kYtNmax || mp > kYtNmax / 2) return false;
     auto kern = k_refine_y_tc;
     const Refusal refuse;
-    if (allow_smem(kern, kYtSmem) != cudaSuccess) return refuse();
+    if (allow_smem(kern, kYtSmem, kYtSmem) != cudaSuccess) return refuse();
     const int nr    = half ? half : n;
     const int ntile = (nr + kYtM - 1) / kYtM;
     kern<<<batch * ntile, kYtNT, kYtSmem, s>>>(H, n, ld, mstride, X32, m, mp, N, reinterpret_cast<float4*>(work), ystride,

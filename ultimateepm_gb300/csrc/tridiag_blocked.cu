@@ -673,6 +673,7 @@ __global__ void __launch_bounds__(kBlkNT, 1)
 
 int tridiag_blocked_max_n() { return kBlkNT; }
 
+constexpr size_t kBlkSmemMost = 227 * 1024 - 64;  // less its static shared memory (48 bytes)
 template <typename S>
 bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq,
                             int* status, int batch, cudaStream_t s, bool tensor_cores) {
@@ -681,12 +682,12 @@ bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>:
     int nc = 0;
     if (tensor_cores && ST<S>::cplx)
         for (int w : {64, 48, 32})
-            if (!nc && BlkSmem<S>::bytes_tc(n, w) <= 227 * 1024) nc = w;
+            if (!nc && BlkSmem<S>::bytes_tc(n, w) <= kBlkSmemMost) nc = w;
     const size_t smem = nc ? BlkSmem<S>::bytes_tc(n, nc) : BlkSmem<S>::bytes(n);
-    if (smem > 227 * 1024) return false;
+    if (smem > kBlkSmemMost) return false;
     auto kern = k_tridiag_blocked<S>;
     const Refusal refuse;
-    if (allow_smem(kern, smem) != cudaSuccess) return refuse();
+    if (allow_smem(kern, smem, kBlkSmemMost) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(NT, MINB)
 template <typename S, int NT, int MINB>
 bool tri_launch(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, int* status, int batch, cudaStream_t s) {
     int nres = n;
-    while (nres > 2 && TriLayout<S>(n, nres, NT).total > kTriSmem - 1024) --nres;
+    while (nres > 2 && TriLayout<S>(n, nres, NT).total > kMaxDynamicSmem) --nres;
     const size_t smem = TriLayout<S>(n, nres, NT).total;
     auto         kern = nres == n ? k_tridiag_tri<S, NT, MINB, false> : k_tridiag_tri<S, NT, MINB, true>;
     const Refusal refuse;

@@ -20,14 +20,17 @@ struct Refusal {
 };
 
 // The dynamic shared memory that a CTA may take: 227 KB, less what the kernels hold as static shared memory (800 bytes
-// at most).
+// at most; k_refine_y_tc, 2 KB, and k_tridiag_blocked name limits of their own).
 constexpr size_t kMaxDynamicSmem = 226 * 1024;
-// Lets a kernel be launched with smem bytes of dynamic shared memory. Without asking it gets 48 KB together with its
-// static shared memory.
+// Lets a kernel be launched with smem bytes of dynamic shared memory, most at the most. Without asking it gets 48 KB
+// together with its static shared memory. The limit belongs to the kernel in the whole process, and another thread
+// may be about to launch it at another size: every call sets the same one, so that none takes from another what it
+// relies on.
 template <typename K>
-cudaError_t allow_smem(K kern, size_t smem) {
+cudaError_t allow_smem(K kern, size_t smem, size_t most = kMaxDynamicSmem) {
     if (smem <= 47 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 void count_launch(int n = 1);
