@@ -233,7 +233,7 @@ void launch_backtransform(const S* H, int n, int ld, size_t mstride, const S* tq
                           cx<typename ST<S>::R>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
                           int batch, cudaStream_t s, int lanes) {
     constexpr bool CX   = sizeof(S) == 2 * sizeof(typename ST<S>::R);
-    const int      tmax = CX ? 24 : 32;  // rows per lane within the register budget
+    const int      tmax = CX ? kBtCplxRows : kBtRealRows;
     if (lanes != 8 && lanes != 16 && lanes != 32) lanes = 0;
     if (lanes && (n + lanes - 1) / lanes > tmax) lanes = 0;
     if (!lanes) lanes = (n + 7) / 8 <= tmax ? 8 : (n + 15) / 16 <= tmax ? 16 : 32;
@@ -265,24 +265,27 @@ UEPM_BT_INST(cx<double>)
 UEPM_BT_INST(cx<float>)
 #undef UEPM_BT_INST
 
-// Quaternion matrices: at most 12 quaternion rows per lane (48 register words), and orders to 256.
+// Quaternion matrices: at most kBtQuatRows quaternion rows per lane (48 register words), and orders to 256.
 template <typename T>
 void launch_backtransform_quat(const qt<T>* H, int n, int ld, size_t mstride, const qt<T>* tq, const T* z, int nz, int nb,
                                cx<T>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
-                               int batch, cudaStream_t s) {
+                               int batch, cudaStream_t s, int lanes) {
+    if (lanes != 8 && lanes != 16 && lanes != 32) lanes = 0;
+    if (lanes && (n + lanes - 1) / lanes > kBtQuatRows) lanes = 0;
+    if (!lanes) lanes = (n + 7) / 8 <= kBtQuatRows ? 8 : (n + 15) / 16 <= kBtQuatRows ? 16 : 32;
 #define UEPM_BTQ(L_, T_) bt_launch<qt<T>, L_, T_>(H, n, ld, mstride, tq, z, nz, Xout, P, d_k, d_G, grad, batch, s, nb)
-    if (n <= 96) UEPM_BTQ(8, 12);
-    else if (n <= 144) UEPM_BTQ(16, 9);
-    else if (n <= 192) UEPM_BTQ(16, 12);
+    if (lanes == 8) UEPM_BTQ(8, 12);
+    else if (lanes == 16 && n <= 144) UEPM_BTQ(16, 9);
+    else if (lanes == 16) UEPM_BTQ(16, 12);
     else UEPM_BTQ(32, 8);
 #undef UEPM_BTQ
 }
 template void launch_backtransform_quat<float>(const qt<float>*, int, int, size_t, const qt<float>*, const float*, int, int,
                                                cx<float>*, const DevParams&, const double*, const int*, double*, int,
-                                               cudaStream_t);
+                                               cudaStream_t, int);
 template void launch_backtransform_quat<double>(const qt<double>*, int, int, size_t, const qt<double>*, const double*, int,
                                                 int, cx<double>*, const DevParams&, const double*, const int*, double*,
-                                                int, cudaStream_t);
+                                                int, cudaStream_t, int);
 
 __global__ void k_pair_values(const double* __restrict__ ev, int nz, double* __restrict__ E, int nb, int total) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -307,7 +307,8 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
                     launch_invit<double>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
                 }
                 ProfScope p(ctx, s, KK_BACKTRANSFORM);
-                launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, P, kk, ctx->d_G, gr, c, s);
+                launch_backtransform_quat<double>(HQ, N, N, qs, tq, z, nz, nb, Xo, P, kk, ctx->d_G, gr, c, s,
+                                                  ctx->tune.vector_lanes);
             }
         }
         return UEPM_OK;
@@ -394,7 +395,8 @@ int run_chunk(uepm_ctx* ctx, const Form& f, const Layout& L, char* ws, const dou
             launch_invit<float>(d, e, ev, nz, N, nz, work, z, st, c, s, ctx->tune.max_iter);
         }
         ProfScope p(ctx, s, KK_BACKTRANSFORM);
-        launch_backtransform_quat<float>(HQ, N, N, qs, qq, z, nz, m, X32, P, kk, ctx->d_G, nullptr, c, s);
+        launch_backtransform_quat<float>(HQ, N, N, qs, qq, z, nz, m, X32, P, kk, ctx->d_G, nullptr, c, s,
+                                         ctx->tune.vector_lanes);
     } else {
     {
         ProfScope p(ctx, s, KK_TRIDIAG32);

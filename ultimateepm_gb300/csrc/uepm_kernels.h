@@ -145,7 +145,9 @@ void launch_backtransform(const S* H, int n, int ld, size_t mstride, const S* tq
 template <typename T>
 void launch_backtransform_quat(const qt<T>* H, int n, int ld, size_t mstride, const qt<T>* tq, const T* z, int nz, int nb,
                                cx<T>* Xout, const DevParams& P, const double* d_k, const int* d_G, double* grad,
-                               int batch, cudaStream_t s);
+                               int batch, cudaStream_t s, int lanes = 0);
+// Rows per lane that the register budget allows: a requested lane count is honoured where its rows fit.
+constexpr int kBtRealRows = 32, kBtCplxRows = 24, kBtQuatRows = 12;
 // The nf scalar levels, vectors ([batch][nf][N]) and gradients of H = diag(h, h) as nb bands for both spins:
 // band 2 q is level q with spin up (x, 0), band 2 q + 1 with spin down (0, x). X, g and their outputs may be null.
 void launch_spin_pairs(const double* E, const cx<double>* X, const double* g, int N, int nf, int nb, int batch, double* Eo,
