@@ -43,11 +43,10 @@ def _solve(c, fake):
     ctx = api._Context(ms.materials[c["material"]], api.generate_basis_vectors(c["shells"])[:c.get("plane_waves")], c.get("nl", False), c.get("soc", False),
                        N.UEPM_PREC_MIXED if c.get("mixed") else N.UEPM_PREC_FP64)
     N.check(N.load().uepm_ctx_set_tuning(ctx.h, C.byref(N.UepmTuning(**c.get("tuning", {})))))
+    fake.fake_clear()
     if "autotune" in c:
         N.check(N.load().uepm_ctx_autotune(ctx.h, c["bands"], N.UEPM_WANT_VALUES, c["autotune"], None))
     fake.fake_refuse(c.get("refuse", "").encode())
-    if "autotune" not in c:
-        fake.fake_clear()
     error = None
     try:
         ctx.solve(np.full((c["k"], 3), 0.1), c["bands"], vectors=c.get("vectors", False))

@@ -33,3 +33,20 @@ def test_every_lane_count_gives_the_same_levels(gpu, oracle, mats, shells):
             ctx.close()
             assert not st.any() and np.abs(E - ref).max() <= tol
             assert max(np.abs(x.conj() @ x.T - np.eye(9)).max() for x in X) <= 1e-8
+
+
+def test_the_autotuner_times_what_changes_the_solve(native, tmp_path):
+    """Shapes timed (three solves each; every shape takes the same time here, so the first stands): the automatic one, the
+    reductions, and of the other fields those that the automatic reduction takes."""
+    ge, inp, si = dict(material="Ge", nl=True, soc=True), dict(material="InP", nl=True), dict(material="Si")
+    want = [(dict(ge, shells=8, mixed=True), 1 + 5 + 3),      # quaternion 89 in shared memory: lanes of 8, 16, 32
+            (dict(ge, shells=10, mixed=True), 1 + 5 + 2),     # 137: lanes of 16, 32
+            (dict(ge, shells=8), 1 + 2 + 5),                  # FP64, global memory: CTAs per SM; no vectors, no lanes
+            (dict(inp, shells=9, mixed=True), 1 + 5 + 3),     # complex 113 in registers
+            (dict(inp, shells=12, mixed=True), 1 + 5 + 3),    # complex 181, triangular
+            (dict(inp, shells=11, mixed=True), 1 + 5 + 5 + 3),  # complex 169, deferred
+            (dict(si, shells=12, mixed=True), 1 + 5 + 3),     # real 181 in registers
+            (dict(si, shells=13, mixed=True), 1 + 5 + 5 + 3)]  # real 229, deferred
+    for (case, shapes), (error, launches, _) in zip(want, fake_runtime.run(tmp_path, *[dict(c, bands=4, k=1, autotune=200) for c, _ in want])):
+        solves = sum("k_rows" in x[0] for x in launches) - 1  # the solve itself
+        assert error is None and solves == 3 * shapes, (case, solves)

@@ -186,28 +186,34 @@ int uepm_ctx_autotune(uepm_ctx* ctx, int nb, uint32_t want, size_t sample_k, voi
     rc               = timed(&best_ms);
     // candidates per field, tried one field at a time from the current best
     const bool mixed = ctx->precision == UEPM_PREC_MIXED;
-    const int  tmax  = ctx->real ? 32 : 24;
-    const bool regok = mixed && ctx->real && ctx->n <= tridiag_reg_max_n();
-    const int  es    = mixed ? (ctx->real ? 4 : 8) : (ctx->real ? 8 : 16);  // bytes of a reduced element
-    std::vector<int> chunks, reds, ctas, lanes, clusters;
-    for (int c : {256, 512, 1024, 2048, 4096, 8192})
-        if ((size_t)c < sample_k) chunks.push_back(c);
-    reds = mixed ? std::vector<int>{2, 3, 4, 5, 6} : std::vector<int>{2, 3};  // 4, 5, 6: FP32 only
-    ctas = {1, 2, 4, 6, 8};
-    for (int c : {2, 4, 8, 16})
-        if ((size_t)es * ctx->n * ((ctx->n + c - 1) / c) <= (200u << 10)) clusters.push_back(c);
-    if (mixed || wv || wg)
-        for (int l : {8, 16, 32})
-            if ((ctx->n + l - 1) / l <= tmax) lanes.push_back(l);
+    const int  es    = mixed ? (ctx->real ? 4 : 8) : (ctx->real ? 8 : 16);  // bytes of an element that reduction 3 spreads
+    // Only what changes the solve: a candidate that runs the same kernels could be kept for its timing's noise.
+    auto candidates = [&](int f) {
+        ctx->tune           = best;
+        const SolveShape sh = solve_shape(ctx);
+        std::vector<int> v;
+        if (f == 0) {
+            for (int c : {256, 512, 1024, 2048, 4096, 8192})
+                if ((size_t)c < sample_k) v.push_back(c);
+        } else if (f == 1) {
+            v = mixed ? std::vector<int>{2, 3, 4, 5, 6} : std::vector<int>{2, 3};  // 4, 5, 6: FP32 only
+        } else if (f == 2) {
+            if (sh.takes_ctas) v = {1, 2, 4, 6, 8};
+        } else if (f == 3) {
+            if (best.reduction == 3)
+                for (int c : {2, 4, 8, 16})
+                    if ((size_t)es * ctx->n * ((ctx->n + c - 1) / c) <= (200u << 10)) v.push_back(c);
+        } else if (mixed || wv || wg) {
+            for (int l : {8, 16, 32})
+                if ((sh.n + l - 1) / l <= (sh.quat ? kBtQuatRows : sh.real ? kBtRealRows : kBtCplxRows)) v.push_back(l);
+        }
+        return v;
+    };
     auto field_of = [](uepm_tuning& t, int f) -> int32_t& {
         return f == 0 ? t.chunk : f == 1 ? t.reduction : f == 2 ? t.ctas_per_sm : f == 3 ? t.cluster : t.vector_lanes;
     };
     for (int field = 0; field < 5 && !rc; ++field) {
-        std::vector<int> cand = field == 0 ? chunks : field == 1 ? reds : field == 2 ? ctas : field == 3 ? clusters : lanes;
-        // ctas_per_sm matters only for the global-memory kernel, cluster only for the cluster kernel
-        if (field == 2 && best.reduction == 3) continue;
-        if (field == 3 && best.reduction != 3 && !(best.reduction == 0 && !ctx->real)) continue;
-        for (int v : cand) {
+        for (int v : candidates(field)) {
             uepm_tuning t    = best;
             field_of(t, field) = v;
             ctx->tune        = t;

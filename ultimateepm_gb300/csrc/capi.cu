@@ -455,6 +455,13 @@ double reduction_cost(const uepm_ctx* ctx) {
     const double N = f.quat ? ctx->N : f.n;
     return N * N * N * (f.quat ? 16.0 : f.real ? 1.0 : 4.0);
 }
+SolveShape solve_shape(const uepm_ctx* ctx) {
+    const Form f     = form_of(ctx);
+    const bool mixed = ctx->precision == UEPM_PREC_MIXED;
+    const int  n     = f.quat ? ctx->N : f.n;
+    // quaternions: the FP32 reduction works in shared memory (tridiag_tri.cu), the FP64 one in global memory
+    return {n, f.real, f.quat, f.quat ? !mixed : tridiag_takes_ctas(mixed, !f.real, n, ctx->tune.reduction)};
+}
 int solve_form(const uepm_ctx* ctx) {
     return ctx->force_cx ? 0 : ctx->decoupled ? (ctx->scalar_real ? 3 : 1) : ctx->quat_h ? 2 : 0;
 }

@@ -103,6 +103,13 @@ double reduction_cost(const uepm_ctx* ctx);
 // The form that an automatic solve of the context works on (0: the matrix itself, 1 or 3: complex or real scalar,
 // 2: quaternion): part of the key under which tunings are shared.
 int solve_form(const uepm_ctx* ctx);
+// What a solve with the context's tuning works on, as far as the tuning's fields depend on it: the order and the
+// scalars of the reduced matrix, and whether its reduction takes ctas_per_sm.
+struct SolveShape {
+    int  n;
+    bool real, quat, takes_ctas;
+};
+SolveShape solve_shape(const uepm_ctx* ctx);
 uint64_t launches_total();
 void     uncount_launches(uint64_t n);
 

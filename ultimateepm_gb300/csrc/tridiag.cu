@@ -617,6 +617,16 @@ void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, t
     else tridiag_pick<S, 16>(H, n, ld, mstride, d, e, tq, status, batch, s, ctas_per_sm);
 }
 
+// Of launch_tridiag's choices the kernels of this file that work in global memory.
+bool tridiag_takes_ctas(bool f32, bool cplx, int n, int variant) {
+    if (variant == 3) return false;
+    if (!f32 || variant == 4 || variant == 5) return true;
+    if (variant == 6) return false;
+    if (variant == 0) return cplx ? n > tridiag_reg_max_n(true) && n < 175 : n > tridiag_reg_max_n() && n < 300;
+    if (variant == 1 && !cplx && n <= tridiag_reg_max_n()) return false;
+    return cplx ? !use_smem<cx<float>>(n) : !use_smem<float>(n);
+}
+
 template void launch_tridiag<cx<double>>(cx<double>*, int, int, size_t, double*, double*, cx<double>*, int*, int, cudaStream_t, int, int, int, bool);
 template void launch_tridiag<cx<float>>(cx<float>*, int, int, size_t, float*, float*, cx<float>*, int*, int, cudaStream_t, int, int, int, bool);
 template void launch_tridiag<double>(double*, int, int, size_t, double*, double*, double*, int*, int, cudaStream_t, int, int, int, bool);

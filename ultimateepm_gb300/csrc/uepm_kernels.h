@@ -79,6 +79,8 @@ template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant = 0, int ctas_per_sm = 0, int cluster = 0,
                     bool tensor_cores = true);
+// Whether launch_tridiag's choice takes ctas_per_sm.
+bool tridiag_takes_ctas(bool f32, bool cplx, int n, int variant);
 // tridiag_wide.cu: the FP64 reduction with a cluster of CTAs per matrix, for few matrices (false, with nothing
 // launched, where that does not pay).
 template <typename S>
