@@ -9,25 +9,34 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")
 
 
+def kernels(tmp_path):
+    """The kernels that the library holds."""
+    return json.loads(_child(tmp_path, "kernels"))
+
+
 def run(tmp_path, *cases):
     """A case: material, shells, bands, k, and optionally plane_waves (the first so many of the basis), nl, soc, mixed,
     vectors, tuning, autotune, refuse. Returns for each its error
     (None: it was solved), its launches (kernel, grid, threads, shared memory) and the shared-memory limits set."""
+    out = []
+    for error, log in json.loads(_child(tmp_path, json.dumps(cases))):
+        lines = [x.split() for x in log.splitlines()]
+        out.append((error, [(x[1], *map(int, x[2:])) for x in lines if x[0] == "launch"],
+                    [(x[1], int(x[2])) for x in lines if x[0] == "smem"]))
+    return out
+
+
+def _child(tmp_path, what):
     from ultimateepm_gb300 import build
 
     lib = os.path.join(str(tmp_path), "libfake_cudart.so")
     if not os.path.exists(lib):
         inc = os.path.join(build._cuda_home(), "include")
         subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + inc, SRC, "-o", lib], check=True)
-    r = subprocess.run([sys.executable, os.path.abspath(__file__), json.dumps(cases)], env=dict(os.environ, LD_PRELOAD=lib, PYTHONPATH=ROOT),
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), what], env=dict(os.environ, LD_PRELOAD=lib, PYTHONPATH=ROOT),
                        capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
-    out = []
-    for error, log in json.loads(r.stdout):
-        lines = [x.split() for x in log.splitlines()]
-        out.append((error, [(x[1], *map(int, x[2:])) for x in lines if x[0] == "launch"],
-                    [(x[1], int(x[2])) for x in lines if x[0] == "smem"]))
-    return out
+    return r.stdout
 
 
 def _solve(c, fake):
@@ -63,4 +72,11 @@ if __name__ == "__main__":
 
     fk = ctypes.CDLL(None)
     fk.fake_log.restype = ctypes.c_char_p
-    print(json.dumps([_solve(c, fk) for c in json.loads(sys.argv[1])]))
+    fk.fake_kernels.restype = ctypes.c_char_p
+    if sys.argv[1] == "kernels":
+        from ultimateepm_gb300 import _native
+
+        _native.load()
+        print(json.dumps(fk.fake_kernels().decode().split()))
+    else:
+        print(json.dumps([_solve(c, fk) for c in json.loads(sys.argv[1])]))

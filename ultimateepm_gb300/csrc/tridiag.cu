@@ -560,7 +560,7 @@ void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, t
             launch_tridiag_reg(H, n, ld, mstride, d, e, tq, status, batch, s);
             return;
         }
-        if (variant == 0 && n >= 175 && n <= 230 && launch_tridiag_tri<S>(H, n, ld, mstride, d, e, tq, status, batch, s))
+        if (variant == 0 && n >= kTriMinCplx && n <= kTriMaxCplx && launch_tridiag_tri<S>(H, n, ld, mstride, d, e, tq, status, batch, s))
             return;
     }
     if constexpr (std::is_same<S, float>::value) {
@@ -622,7 +622,7 @@ bool tridiag_takes_ctas(bool f32, bool cplx, int n, int variant) {
     if (variant == 3) return false;
     if (!f32 || variant == 4 || variant == 5) return true;
     if (variant == 6) return false;
-    if (variant == 0) return cplx ? n > tridiag_reg_max_n(true) && n < 175 : n > tridiag_reg_max_n() && n < 300;
+    if (variant == 0) return cplx ? n > tridiag_reg_max_n(true) && n < kTriMinCplx : n > tridiag_reg_max_n() && n < 300;
     if (variant == 1 && !cplx && n <= tridiag_reg_max_n()) return false;
     return cplx ? !use_smem<cx<float>>(n) : !use_smem<float>(n);
 }

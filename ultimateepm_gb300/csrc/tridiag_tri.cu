@@ -436,7 +436,10 @@ bool tri_launch(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, 
     int nres = n;
     while (nres > 2 && TriLayout<S>(n, nres, NT).total > kMaxDynamicSmem) --nres;
     const size_t smem = TriLayout<S>(n, nres, NT).total;
-    auto         kern = nres == n ? k_tridiag_tri<S, NT, MINB, false> : k_tridiag_tri<S, NT, MINB, true>;
+    auto         kern = k_tridiag_tri<S, NT, MINB, false>;
+    if constexpr (MINB == 1) {  // where more CTAs share an SM their triangles fit as they are
+        if (nres < n) kern = k_tridiag_tri<S, NT, MINB, true>;
+    }
     const Refusal refuse;
     if (allow_smem(kern, smem) != cudaSuccess) return refuse();
     int dev = 0, sms = 0, fit = 0;
@@ -452,16 +455,20 @@ bool tri_launch(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, 
 }  // namespace
 
 // 16 warps per SM at the kernel's 128 registers: CTAs of 128 threads where four fit an SM's shared memory
-// (N <= 74), of 256 where two do (N <= 109), else one of 512.
+// (N <= 74), of 256 where two do (N <= 109), else one of 512. Complex matrices come at orders that fill an SM
+// (launch_tridiag says why those): CTAs of 512 alone.
 template <typename S>
 bool launch_tridiag_tri(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, int* status, int batch,
                         cudaStream_t s) {
-    if (n < 1 || n > 512) return false;
-    const size_t sm = kTriSmem;
-    if (n <= 256 && 4 * (TriLayout<S>(n, n, 128).total + 2048) <= sm)
-        return tri_launch<S, 128, 4>(H, n, ld, mstride, d, e, tq, status, batch, s);
-    if (2 * (TriLayout<S>(n, n, 256).total + 2048) <= sm)
-        return tri_launch<S, 256, 2>(H, n, ld, mstride, d, e, tq, status, batch, s);
+    if constexpr (is_quat<S>::value) {
+        if (n < 1 || n > 256) return false;
+        if (4 * (TriLayout<S>(n, n, 128).total + 2048) <= kTriSmem)
+            return tri_launch<S, 128, 4>(H, n, ld, mstride, d, e, tq, status, batch, s);
+        if (2 * (TriLayout<S>(n, n, 256).total + 2048) <= kTriSmem)
+            return tri_launch<S, 256, 2>(H, n, ld, mstride, d, e, tq, status, batch, s);
+    } else {
+        if (n < kTriMinCplx || n > kTriMaxCplx) return false;
+    }
     return tri_launch<S, 512, 1>(H, n, ld, mstride, d, e, tq, status, batch, s);
 }
 template bool launch_tridiag_tri<cx<float>>(cx<float>*, int, int, size_t, float*, float*, cx<float>*, int*, int,

@@ -102,8 +102,9 @@ int tridiag_blocked_max_n();
 template <typename S>
 bool launch_tridiag_blocked(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq,
                             int* status, int batch, cudaStream_t s, bool tensor_cores);
-// tridiag_tri.cu: the reduction of quaternion (order 1..256) and complex matrices with the lower triangle in
-// shared memory (H: at least the lower triangle, column-major; false when it cannot run).
+// tridiag_tri.cu: the reduction of quaternion (order 1..256) and complex matrices (order kTriMinCplx..kTriMaxCplx)
+// with the lower triangle in shared memory (H: at least the lower triangle, column-major; false when it cannot run).
+constexpr int kTriMinCplx = 175, kTriMaxCplx = 230;
 template <typename S>
 bool launch_tridiag_tri(S* H, int n, int ld, size_t mstride, float* d, float* e, S* tq, int* status, int batch,
                         cudaStream_t s);
