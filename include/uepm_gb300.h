@@ -175,6 +175,13 @@ int uepm_pivot_reciprocal_device(const double* d_q, double pivmin, size_t n, dou
  * values. */
 int uepm_ds_special_device(int fn, const double* d_x, size_t n, double* d_y, void* stream);
 
+/* Diagnostics (no reference counterpart): the scalars of the Householder reductions, from device x [3][n] to
+ * device y [5][n], enqueued on `stream`. fn 0, FP64: of x[0] > 0 the square root y[0], its reciprocal y[1] and the
+ * reciprocal y[2]. fn 1 and 2, FP32 (x rounded to it), real and complex: of the column (alpha; tail), alpha =
+ * x[0] + i x[1] and |tail|^2 = x[2], beta y[0], tau y[1] + i y[2] and 1 / (alpha - beta) y[3] + i y[4]. Lets
+ * tests bound what the kernels refine from hardware approximations. */
+int uepm_reflector_scalars_device(int fn, const double* d_x, size_t n, double* d_y, void* stream);
+
 /* Launch counters (kernels enqueued by this library since load), for launch accounting. */
 uint64_t uepm_kernel_launches(void);
 
