@@ -115,8 +115,12 @@ int uepm_ctx_set_workspace_limit(uepm_ctx* ctx, size_t bytes);
 /* When H(k) is exactly real for the context's material and flags (no SOC, all antisymmetric form
  * factors zero, identical anion/cation nonlocal parameters: elemental diamond-structure crystals),
  * the solve runs real-symmetric kernels, a quarter of the complex arithmetic, with the same results.
- * on != 0 forces the complex kernels (for cross-checks). Returns 1 if the real kernels will run,
- * 0 otherwise. */
+ * Spin-orbit contexts have two forms of their own, of the order N of the basis instead of 2 N:
+ *   quaternion  equal atoms and no antisymmetric form factors (Si, Ge, Sn): every level is a Kramers pair,
+ *               and H(k) is a quaternion matrix;
+ *   scalar      no spin-orbit strength (mu_soc = 0): the scalar matrix, each level for both spins.
+ * on != 0 forces the complex kernels on the whole matrix (for cross-checks), in place of the real ones and
+ * of both these forms. Returns 1 if the real kernels will run, 0 otherwise. */
 int uepm_ctx_force_complex(uepm_ctx* ctx, int on);
 
 /*
@@ -202,7 +206,10 @@ int uepm_measure_peak(int precision, double* tflops);
 
 /* ---- Tuning (no reference counterpart) -------------------------------------------------------
  * Kernel-shape choices of a context. 0 in a field means "automatic":
- *   reduction     the Householder reduction kernel: 1 register-resident (FP32 real matrices, n <= 192),
+ *   reduction     the Householder reduction kernel. Any but 0 reduces H(k) as it stands: spin-orbit contexts
+ *                 that are solved in quaternion or scalar form (uepm_ctx_force_complex) go back to the
+ *                 complex matrix of order 2 N, at several times the cost.
+ *                 1 register-resident (FP32 real matrices, n <= 192),
  *                 2 one CTA per matrix (shared memory where the matrix fits, else global memory with
  *                 a persistent grid), 3 one thread-block cluster per matrix, the matrix spread over
  *                 the cluster's shared memory (orders beyond one SM), 4 one CTA per matrix in global
@@ -211,13 +218,19 @@ int uepm_measure_peak(int precision, double* tflops);
  *                 to the next pass (a read-only pass, then a rank-4 pass: 3 passes per two steps), 6 blocked:
  *                 panels of 16 columns whose updates are applied once per panel, only the lower
  *                 triangle read and written, one matrix per SM (FP32, n <= 512);
- *                 automatic: 1 where it applies, 6 for the FP32 orders 200..512 (real: 300..512), 5 for the other FP32
- *                 matrices, else 2
- *   ctas_per_sm   CTAs per SM of the global-memory reduction (its L2 working set), 1..8
- *   vector_lanes  lanes per eigenvector in the back-transformation: 8, 16 or 32
+ *                 automatic (n the order of the form that is solved): FP32 real matrices in registers to n = 192,
+ *                 5 from there and 6 from 300; FP32 complex ones in registers to n = 144, 5 to 174, on the lower
+ *                 triangle in shared memory to 230, 6 from there; FP32 quaternion ones on the triangle; FP64
+ *                 ones 2, and for at most half as many matrices as SMs (and orders large enough) a cluster
+ *                 of 2, 4 or 8 CTAs per matrix, with the same bits
+ *   ctas_per_sm   CTAs per SM of the reductions in global memory (2 where the matrix does not fit shared memory,
+ *                 4 and 5; their L2 working set), 1..8. The others ignore it. FP64 solves with it set take one CTA
+ *                 per matrix
+ *   vector_lanes  lanes per eigenvector in the back-transformation: 8, 16 or 32, where its rows fit a lane's
+ *                 registers (32 real, 24 complex, 12 quaternion rows per lane), else automatic
  *   chunk         k-points per pipeline pass (smaller keeps H(k) resident in L2 between the
  *                 kernels of a pass), 64..32768
- *   cluster       CTAs per cluster of reduction 3: 2, 4, 8 or 16
+ *   cluster       CTAs per cluster of reduction 3 (the others ignore it): 2, 4, 8 or 16
  *   max_iter      iteration cap (0..1000) of the iterative kernels: bisection steps per phase
  *                 (automatic 64 / 200), inverse-iteration solves per vector (automatic 4 FP32, 5 FP64)
  *                 and projected-Jacobi sweeps (automatic 12). A k-point whose iteration the cap ends
@@ -239,8 +252,8 @@ int uepm_measure_peak(int precision, double* tflops);
  * Every choice gives results within the parity tolerances; a given choice is deterministic.
  * uepm_ctx_autotune times candidate shapes on sample_k seeded random first-zone k-points (coordinate
  * descent over the fields, CUDA events on `stream`) and keeps the fastest; results are cached
- * process-wide per (device, n, real/complex, precision, nb, vectors) so that contexts of the same
- * shape reuse them. It allocates and synchronises: call it before capturing work into a graph. */
+ * process-wide per (device, n, real/complex, form of H(k), precision, nb, vectors) so that contexts of the
+ * same shape reuse them. It allocates and synchronises: call it before capturing work into a graph. */
 typedef struct uepm_tuning {
     int32_t reduction;
     int32_t ctas_per_sm;

@@ -6,7 +6,7 @@
 // Tuning. A context's kernel-shape choices (uepm_tuning) are threaded into its launches. The
 // autotuner times candidate shapes on a seeded sample of first-zone k-points with CUDA events and
 // keeps the fastest, one field at a time (coordinate descent from the automatic choices); the result
-// is cached per (device, n, real/complex, precision, nb, vectors).
+// is cached per (device, n, real/complex, form of H(k), precision, nb, vectors).
 //
 // Batches. Groups of (context, k-points, outputs) are enqueued together: each distinct context on
 // its own stream, forked from and joined back to the caller's stream, so the per-context pipelines

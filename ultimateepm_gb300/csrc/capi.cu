@@ -469,13 +469,14 @@ int solve_form(const uepm_ctx* ctx) {
 // Two lanes: a mixed solve's reduction holds the SMs' registers or shared memory, and the kernels
 // after it (bisection, inverse iteration, the Rayleigh-Ritz products and the small solves) are bound
 // by the latency of short per-matrix chains. Splitting the batch over two streams lets one half's
-// later kernels run beside the other half's reduction. Per solve, one lane against two: Si local
-// n = 137 (register-resident reduction), 2000 k, 16 bands: 2.00 -> 1.89 ms (three and four lanes no
-// faster); 12 bands, Si nonlocal n = 137, 65536 k: 100.8 -> 100.0 ms; InP n = 113 complex: 158.5 ->
-// 155.9; Ge n = 181 real, 32768 k: 151.2 -> 149.2; Ge SOC n = 362, 16 bands, 4000 k: 113.7 -> 111.0
-// (each half in one pass of its own). Results are the same bits (every k-point is solved on its own).
-// FP64 solves keep one stream: two measured 12.5 -> 12.9 ms (Si local, 2000 k), 601.7 -> 604.4 (Ge
-// SOC, 2000 k) and 138.5 -> 131.4 (Ge n = 181 real, 8000 k), no gain overall.
+// later kernels run beside the other half's reduction. Per solve, one lane against two, ms: Si local
+// n = 137, 16 bands, 1024 k 0.836 -> 0.811, 2000 k 1.476 -> 1.435, 8000 k 5.21 -> 5.14; Si nonlocal n = 137, 12
+// bands, 1024 k 1.162 -> 1.115, 20000 k 18.62 -> 18.18; InP n = 113 complex, 1024 k 1.650 -> 1.610, 20011 k
+// 28.07 -> 28.01; Ge n = 181 real, 1024 k 2.02 -> 1.94, 10007 k 17.38 -> 17.26; Ge SOC (quaternion 181), 16 bands,
+// 1024 k 12.25 -> 11.95, 3001 k 34.78 -> 34.45; GaAs SOC n = 178, 1024 k 7.24 -> 6.92, 338 (blocked reduction),
+// 1500 k 36.3 -> 35.9; Si SOC (scalar 137), 4000 k 2.24 -> 2.21. Results are the same bits (every k-point is solved
+// on its own). FP64 solves keep one stream: two measured 10.13 -> 9.89 (Si local, 2000 k), 21.46 -> 21.15 (InP, 2000
+// k), 74.1 -> 73.3 (Ge SOC, 500 k) and 52.1 -> 54.1 (Ge n = 181 real, 4000 k), no gain for all.
 constexpr size_t kLaneMinK = 1024;
 static bool lanes_pay(const uepm_ctx* ctx, size_t nk) { return ctx->precision == UEPM_PREC_MIXED && nk >= kLaneMinK; }
 

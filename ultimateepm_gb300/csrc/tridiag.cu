@@ -18,7 +18,7 @@
 //     p = A22 v is a plain row-by-lane product with per-lane accumulators and no cross-lane
 //     reductions (4 FMA per element, complex);
 //   * chunk loops have warp-uniform bounds, so fully masked chunks are skipped, not issued;
-//   * the Householder scalars (sqrt, reciprocals) are computed once per CTA by one thread.
+//   * the Householder scalars (sqrt, reciprocals) are computed once per CTA, by its first warp.
 // Per step: 4 m^2 FMA for the product + 4 m^2 for the lower-triangle update (complex), i.e. the
 // 16/3 n^3 algorithmic flops (4/3 n^3 for real symmetric matrices). The matrix lives in a per-k HBM
 // workspace; the 129 MB L2 holds the working set of the resident CTAs.
@@ -482,7 +482,7 @@ static void tridiag_launch_t(S* H, int n, int ld, size_t mstride, typename ST<S>
     int grid = batch;
     if (!SMEM) {
         // automatic: keep the matrices in flight within ~120 MB so that they stay in the 129 MB L2
-        // (FP64 at n = 137: 5 per SM, 13.1 ms for 2000 matrices against 14.1 at 4 and 14.5 at 6), but
+        // (FP64 at n = 137: 5 per SM; a solve of 2000 k takes 10.12 ms with 5 and 10.16 with 4), but
         // never below 4 CTAs per SM: for large (complex / spin-orbit) matrices, latency hiding wins
         // over L2 residency (measured 1.5-2x over 1 CTA per SM at n = 178..458, FP32)
         const size_t bytes  = sizeof(S) * (size_t)n * n;

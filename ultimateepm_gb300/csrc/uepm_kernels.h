@@ -70,11 +70,12 @@ void launch_assemble(const DevParams& P, const cx<double>* Vloc, const double2* 
 // thread-block cluster per matrix (tridiag_cluster.cu), 4 one CTA per matrix in global memory with
 // each step's update fused into the next step's product (FP32, n <= 512), 5 the same with every
 // other update deferred to the next pass, 6 blocked (panels of 16 columns, lower triangle only, one
-// matrix per SM, tridiag_blocked.cu; FP32, n <= 512). Automatic: 1 where it applies, for
-// FP32 complex orders 175..230 the triangular kernel (tridiag_tri.cu) and 231..512 6, for real orders
-// 300..512 6, 5 for the other FP32 matrices, else 2.
-// ctas_per_sm (0: automatic) caps the persistent grid of the global-memory kernels; cluster (0:
-// automatic) is the cluster size of variant 3.
+// matrix per SM, tridiag_blocked.cu; FP32, n <= 512). Automatic: FP32 in registers to
+// tridiag_reg_max_n(complex), for complex orders 175..230 the triangular kernel (tridiag_tri.cu) and from 231
+// 6, for real orders from 300 6, else 5; FP64 2, with a cluster of CTAs per matrix for few matrices
+// (tridiag_wide.cu).
+// ctas_per_sm (0: automatic) caps the persistent grid of the global-memory kernels (tridiag_takes_ctas); cluster
+// (0: automatic) is the cluster size of variant 3.
 template <typename S>
 void launch_tridiag(S* H, int n, int ld, size_t mstride, typename ST<S>::R* d, typename ST<S>::R* e, S* tq, int* status,
                     int batch, cudaStream_t s, int variant = 0, int ctas_per_sm = 0, int cluster = 0,
